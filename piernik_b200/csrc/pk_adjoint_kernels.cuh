@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sweep_fused_rec(Geom g, Tile tl,
 {
     extern __shared__ double smem[];
     unsigned status = 0;
-    fused_tile<PH, true>(g, tl, blockIdx.x * tl.P, blockIdx.y * tl.L, blockIdx.z, uin, uout, pp, sp, dl, apply_fac, smem,
+    fused_tile<PH, MAXT, true>(g, tl, blockIdx.x * tl.P, blockIdx.y * tl.L, blockIdx.z, uin, uout, pp, sp, dl, apply_fac, smem,
                          status, ustar, flags);
     flush_status(status, gstatus);
 }

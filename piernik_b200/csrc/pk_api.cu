@@ -818,7 +818,7 @@ int build_batch(pk_ctx* h)
             int P = SV_T[sv] / T;
             if (P > face) P = face;
             StageList& sl = h->sbatch[dir][b.level];
-            sl.smem = std::max(sl.smem, (size_t)3 * h->nplanes * P * T * sizeof(double));
+            sl.smem = (size_t)3 * h->nplanes * SV_T[sv] * sizeof(double);
             for (int q = 0; q < face; q += P) items[b.level].push_back(StageItem{i, q, 0, P});
         }
         for (int L = 0; L <= maxl; ++L) {

@@ -154,6 +154,30 @@ PK_PHYS double slope_interior(int lim, double dl, double dr)
     return (s * 0.5) * m;
 }
 
+// half * f_limiter(q) of an interior cell for a limiter known at compile time
+// (dq_interp = half * f_limiter(q), interpolations.F90:170-204).  Bit for bit
+// 0.5 * slope_interior(LIM, dl, dr): the signs s of minmod, moncen and superbee
+// are -2, 0 or 2, so ((s * m) * 0.5) * 0.5 rounds once, as (s / 4) * m does (for
+// limited differences below 2^1023; s = 0 keeps the +0, and the NaN of 0 * inf),
+// and min(2a, 2b) = 2 min(a, b) exactly.
+template <int LIM>
+PK_PHYS double half_slope(double dl, double dr)
+{
+    if (LIM == L_VANLEER) {
+        const double dcen = dl * dr;
+        return 0.5 * ((dcen > 0.0) ? (2.0 * dcen) / (dl + dr) : 0.0);
+    }
+    const double adl = fabs(dl), adr = fabs(dr);
+    double m;
+    if (LIM == L_MINMOD) m = f_min(adl, adr);
+    else if (LIM == L_MONCEN) m = f_min(2.0 * f_min(adl, adr), 0.5 * fabs(dl + dr));
+    else m = (adl > adr) ? f_min(adl, 2.0 * adr) : f_min(2.0 * adl, adr);
+    const unsigned long long bl = f_bits(dl), br = f_bits(dr);
+    const double s = f_from_bits(((long long)(bl ^ br) < 0) ? 0ULL
+                                                            : ((bl & 0x8000000000000000ULL) | 0x3fe0000000000000ULL));
+    return s * m;
+}
+
 // WENO3 face states of cell c from q(c-1), q(c), q(c+1) (interpolations.F90:
 // 210-337, Yamaleev & Carpenter 2009): ql = the left state of the right face,
 // qr = the right state of the left face, in the reference's operation order.
@@ -549,54 +573,6 @@ PK_PHYS void riemann(const double (&ql)[PH::NV], const double (&qr)[PH::NV], dou
 #pragma unroll
         for (int c = 0; c < 5; ++c)
             if (c < PH::ncomp(PH::kind(f))) fx[b + c] = fv[c];
-    }
-}
-
-// The same for a tile in shared memory: left states at L[v*PT + me], right
-// states at R[v*PT + me + st], fluxes written to F[v*PT + me].  Each fluid's
-// states are loaded just before its solve, so the register footprint does not
-// grow with the number of fluids.
-template <class PH>
-PK_DEV void riemann_tile(const double* __restrict__ L, const double* __restrict__ R, double* __restrict__ F, int PT,
-                         int me, int st, double ch, const PhysParams& pp)
-{
-    double blv[3] = {0.0, 0.0, 0.0}, brv[3] = {0.0, 0.0, 0.0};
-    if (PH::MHD) {
-        const double bxl = L[PH::IB * PT + me], bxr = R[PH::IB * PT + me + st];
-        const double psl = L[(PH::IB + 3) * PT + me], psr = R[(PH::IB + 3) * PT + me + st];
-        F[(PH::IB + 3) * PT + me] = ((ch * ch) * 0.5) * ((bxr + bxl) - (psr - psl) / ch);   // hlld.F90:229
-        F[PH::IB * PT + me] = 0.5 * ((psr + psl) - ch * (bxr - bxl));                      // :230
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            blv[c] = L[(PH::IB + c) * PT + me];
-            brv[c] = R[(PH::IB + c) * PT + me + st];
-        }
-    }
-#pragma unroll
-    for (int f = 0; f < PH::NFL; ++f) {
-        const int b = PH::beg(f);
-        const int nc = PH::ncomp(PH::kind(f));
-        double ul[5] = {0, 0, 0, 0, 0}, ur[5] = {0, 0, 0, 0, 0}, fv[5];
-#pragma unroll
-        for (int c = 0; c < 5; ++c)
-            if (c < nc) {
-                ul[c] = L[(b + c) * PT + me];
-                ur[c] = R[(b + c) * PT + me + st];
-            }
-        if (PH::MHD) {
-            const double zero[3] = {0.0, 0.0, 0.0};
-            double bf[2];
-            hlld_iface(PH::has_en(f), pp.gam[f], ul, ur, PH::magn(f) ? blv : zero, PH::magn(f) ? brv : zero, fv, bf);
-            if (PH::magn(f)) {
-                F[(PH::IB + 1) * PT + me] = bf[0];
-                F[(PH::IB + 2) * PT + me] = bf[1];
-            }
-        } else {
-            hllc_iface(PH::has_en(f), pp.gam[f], ul, ur, fv);
-        }
-#pragma unroll
-        for (int c = 0; c < 5; ++c)
-            if (c < nc) F[(b + c) * PT + me] = fv[c];
     }
 }
 

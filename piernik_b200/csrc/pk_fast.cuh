@@ -395,27 +395,34 @@ PK_DEV void hllc_iface_fast(bool has_energy, double gamma, double rgam_1, const 
     }
 }
 
-}  // namespace pk
-
-namespace pk {
-
-// riemann_tile (pk_device.cuh) with the tolerance-mode solvers: the GLM flux
-// of psi multiplies by 1/ch instead of dividing
-template <class PH>
-PK_DEV void riemann_tile_fast(const double* __restrict__ L, const double* __restrict__ R, double* __restrict__ F,
-                              int PT, int me, int st, double ch, double rch, const PhysParams& pp)
+// riemann_wrap / riemann_wrap_u (hlld.F90:62-155) for the right face of one
+// cell of a tile in shared memory (planes of S doubles): its left state in q
+// (KEEP) or at F[v * S], the right state at R[v * S].  The fluxes go to F[v * S]
+// and, with KEEP, to q.  Each fluid's states are loaded just before its solve.
+// FAST: the tolerance-mode solvers; the GLM flux of psi multiplies by 1/ch
+// instead of dividing.
+template <class PH, int S, bool KEEP, bool FAST>
+PK_DEV void riemann_cell(double (&q)[PH::NV], const double* R, double* F, double ch, const PhysParams& pp)
 {
+    auto left = [&](int v) { return KEEP ? q[v] : F[v * S]; };
+    auto put = [&](int v, double f) {
+        F[v * S] = f;
+        if (KEEP) q[v] = f;
+    };
     double blv[3] = {0.0, 0.0, 0.0}, brv[3] = {0.0, 0.0, 0.0};
     if (PH::MHD) {
-        const double bxl = L[PH::IB * PT + me], bxr = R[PH::IB * PT + me + st];
-        const double psl = L[(PH::IB + 3) * PT + me], psr = R[(PH::IB + 3) * PT + me + st];
-        F[(PH::IB + 3) * PT + me] = ((ch * ch) * 0.5) * ((bxr + bxl) - (psr - psl) * rch);   // hlld.F90:229
-        F[PH::IB * PT + me] = 0.5 * ((psr + psl) - ch * (bxr - bxl));                       // :230
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            blv[c] = L[(PH::IB + c) * PT + me];
-            brv[c] = R[(PH::IB + c) * PT + me + st];
+            blv[c] = left(PH::IB + c);
+            brv[c] = R[(PH::IB + c) * S];
         }
+        const double bxl = blv[0], bxr = brv[0];
+        const double psl = left(PH::IB + 3), psr = R[(PH::IB + 3) * S];
+        double dps;
+        if constexpr (FAST) dps = (psr - psl) * rcp_nr(ch);
+        else dps = (psr - psl) / ch;
+        put(PH::IB + 3, ((ch * ch) * 0.5) * ((bxr + bxl) - dps));                // hlld.F90:229 (Dedner eq. 42)
+        put(PH::IB, 0.5 * ((psr + psl) - ch * (bxr - bxl)));                     // :230
     }
 #pragma unroll
     for (int f = 0; f < PH::NFL; ++f) {
@@ -425,24 +432,29 @@ PK_DEV void riemann_tile_fast(const double* __restrict__ L, const double* __rest
 #pragma unroll
         for (int c = 0; c < 5; ++c)
             if (c < nc) {
-                ul[c] = L[(b + c) * PT + me];
-                ur[c] = R[(b + c) * PT + me + st];
+                ul[c] = left(b + c);
+                ur[c] = R[(b + c) * S];
             }
         if (PH::MHD) {
             const double zero[3] = {0.0, 0.0, 0.0};
+            const double* bl = PH::magn(f) ? blv : zero;
+            const double* br = PH::magn(f) ? brv : zero;
             double bf[2];
-            hlld_iface_fast(PH::has_en(f), pp.gam[f], pp.rgam_1[f], pp.rgam[f], ul, ur, PH::magn(f) ? blv : zero,
-                            PH::magn(f) ? brv : zero, fv, bf);
+            if constexpr (FAST)
+                hlld_iface_fast(PH::has_en(f), pp.gam[f], pp.rgam_1[f], pp.rgam[f], ul, ur, bl, br, fv, bf);
+            else
+                hlld_iface(PH::has_en(f), pp.gam[f], ul, ur, bl, br, fv, bf);
             if (PH::magn(f)) {
-                F[(PH::IB + 1) * PT + me] = bf[0];
-                F[(PH::IB + 2) * PT + me] = bf[1];
+                put(PH::IB + 1, bf[0]);
+                put(PH::IB + 2, bf[1]);
             }
         } else {
-            hllc_iface_fast(PH::has_en(f), pp.gam[f], pp.rgam_1[f], ul, ur, fv);
+            if constexpr (FAST) hllc_iface_fast(PH::has_en(f), pp.gam[f], pp.rgam_1[f], ul, ur, fv);
+            else hllc_iface(PH::has_en(f), pp.gam[f], ul, ur, fv);
         }
 #pragma unroll
         for (int c = 0; c < 5; ++c)
-            if (c < nc) F[(b + c) * PT + me] = fv[c];
+            if (c < nc) put(b + c, fv[c]);
     }
 }
 

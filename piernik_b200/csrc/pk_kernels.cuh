@@ -11,7 +11,7 @@
 // by __syncthreads:
 //   1. utoq          -> Q (primitives)
 //   2. limited slope -> ql in registers, qr of the cell's left face -> R
-//   3. Riemann flux at the cell's right face (own ql, neighbour's R) -> Q
+//   3. Riemann flux at the cell's right face (own ql, neighbour's R) -> F
 //   4. u1 = u0 + dtodx*(F(i-1/2) - F(i+1/2)), internal_sources, floors
 // Which cells do what is decided per thread from its pencil position:
 //   * fused mode (periodic single block): both RK2 stages in one launch over a
@@ -96,19 +96,53 @@ struct Roles {
     bool keep;     // not updated but kept (pencil end cell): u1 = u, then floors
 };
 
-// Shared-memory planes of a tile: Q holds primitives and then face fluxes, L
-// the left state of each cell's right face, R the right state of its left face.
-struct Smem {
-    double* Q;
-    double* L;
-    double* R;
-    int PT;
-};
+// Shared-memory planes of a tile, S doubles per plane (S a compile-time bound
+// on the tile's cells, so that every access is one base register plus an
+// immediate offset): Q the primitives, R the right state of each cell's left
+// face, F the flux through its right face.
+template <class PH, int S>
+PK_PHYS constexpr size_t tile_doubles() { return (size_t)3 * PH::NV * S; }
 
-// One stage of solve() on the tile.  Nothing but the cell's own state w crosses
-// a barrier in registers: primitives and face states live in shared memory and
-// the stage's initial state u0 is re-read (from L2) at the update, so the
-// Riemann solver runs with a small live set.
+// The face states of one cell from its own primitives q and its neighbours'
+// (slots mp, mn) for component planes [V0, V1): q becomes the left state of the
+// cell's right face, the right state of its left face goes to R.  The limiter
+// is uniform over the tile, so the choice is made once for all planes.
+template <int S, int V0, int V1, int NV>
+PK_DEV void limited_faces(int lim, const double* __restrict__ Q, double* __restrict__ R, int me, int mp, int mn, int end,
+                          double (&q)[NV])
+{
+    auto faces = [&](auto half) {
+#pragma unroll
+        for (int v = V0; v < V1; ++v) {
+            const double qc = q[v];
+            double dl = qc - Q[v * S + mp], dr = Q[v * S + mn] - qc;
+            if (end < 0) dl = dr;                             // pencil ends: the reference's one-sided rules
+            if (end > 0) dr = dl;
+            const double dqh = half(dl, dr);                  // dq_interp = half * f_limiter(q)
+            q[v] = qc + dqh;
+            R[v * S + me] = qc - dqh;
+        }
+    };
+    switch (lim) {
+    case L_VANLEER: faces([&](double dl, double dr) { return end == 0 ? half_slope<L_VANLEER>(dl, dr) : 0.0; }); break;
+    case L_MINMOD: faces([](double dl, double dr) { return half_slope<L_MINMOD>(dl, dr); }); break;
+    case L_MONCEN: faces([](double dl, double dr) { return half_slope<L_MONCEN>(dl, dr); }); break;
+    default: faces([](double dl, double dr) { return half_slope<L_SUPERBEE>(dl, dr); }); break;
+    }
+}
+
+// One stage of solve() on the tile, three barriers.  Nothing but the cell's own
+// values crosses a barrier in registers: its primitives (then the left state of
+// its right face) to the slope phase and the solver, its flux to the update;
+// its neighbours' come from the shared planes.  With more than KEEP_NV
+// components the left state and the flux cross in the cell's own slot of F
+// instead (nobody else touches that slot between the barriers), so the register
+// footprint does not grow with the number of fluids.  The stage's initial state
+// u0 is re-read (from L2, or the staged box) at the update.  Q is read between
+// the first two barriers, R between the last two and F after the last, so the
+// next stage may start at once: its first writes to each plane lie at least one
+// barrier behind the last reads.
+//   sm     the planes (tile_doubles<PH, S>() doubles)
 //   w      in: the stage's input state (valid where r.q); out: u1 where r.upd or r.keep
 //   u0src  where u0 (uh / the sweep's input) is read for the update
 //   wsrc   where an unchanged end cell re-reads its state (r.keep)
@@ -126,65 +160,85 @@ struct Smem {
 //          are compiled in their own translation units with contraction on
 //   U0S    u0 comes from shared memory (a staged tile): component plane j of
 //          this cell at u0sm[j * u0st] instead of u0src in global memory
-template <class PH, bool REC = false, bool W3 = false, bool FC = false, bool FAST = false, bool U0S = false>
-PK_DEV void rk_stage(const Smem& sm, int me, int mp, int mn, const Roles& r, double (&w)[PH::NV], const double* u0src,
-                     const double* wsrc, long long off, const Geom& g, double dtodx, double ch,
+//   FLUX   stop after the fluxes: w returns them (where r.flux) instead of u1
+// What bounds it: issue slots and FP64 latency (3625 warp slots per cell and
+// MHD sweep before, of which 1600 FP64).  With run-time plane strides, a limiter
+// switch per component, every value of the cell re-read from shared memory and
+// a fourth barrier, the staged sweeps of a 256^3 MHD block (moncen) took 3.05 ms
+// each bit-exact and 2.19 in the tolerance arithmetic; like this 2.75 and 1.87.
+constexpr int KEEP_NV = 9;
+
+template <class PH, int S, bool REC = false, bool W3 = false, bool FC = false, bool FAST = false, bool U0S = false,
+          bool FLUX = false>
+PK_DEV void rk_stage(double* __restrict__ sm, int me, int mp, int mn, const Roles& r, double (&w)[PH::NV],
+                     const double* u0src, const double* wsrc, long long off, const Geom& g, double dtodx, double ch,
                      const PhysParams& pp, unsigned& status, FloorRec* rec = nullptr,
                      const double* fc_in = nullptr, double* fc_out = nullptr, const double* u0sm = nullptr,
                      int u0st = 0)
 {
     constexpr int NV = PH::NV;
-    const int PT = sm.PT;
+    constexpr bool KEEP = NV <= KEEP_NV;
+    double* const Q = sm;
+    double* const R = sm + NV * S;
+    double* const F = sm + 2 * NV * S;
+    double q[NV];
     if (r.q) {
-        double q[NV];
         if constexpr (FAST) utoq_fast<PH>(w, q, pp);
         else utoq<PH>(w, q, pp);
 #pragma unroll
-        for (int v = 0; v < NV; ++v) sm.Q[v * PT + me] = q[v];
+        for (int v = 0; v < NV; ++v) Q[v * S + me] = q[v];
     }
     __syncthreads();
-    if constexpr (W3) {
-        if (r.slope) {
+    if (r.slope) {
+        if constexpr (!KEEP) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const double qc = sm.Q[v * PT + me];
-            double l = qc, rr = qc;                           // pencil ends: ql(1) = q(1), qr(n-1) = q(n)
-            if (r.end == 0) weno3_faces(sm.Q[v * PT + mp], qc, sm.Q[v * PT + mn], pp.w_epsilon, l, rr);
-            sm.L[v * PT + me] = l;
-            sm.R[v * PT + me] = rr;
+            for (int v = 0; v < NV; ++v) q[v] = Q[v * S + me];
         }
-        }
-    } else if (r.slope) {
+        if constexpr (W3) {
 #pragma unroll
-        for (int v = 0; v < NV; ++v) {
-            const int lim = (PH::MHD && v >= PH::IB) ? pp.limb : pp.lim;
-            const double qc = sm.Q[v * PT + me];
-            double s;
-            if (r.end < 0) s = slope_end(lim, sm.Q[v * PT + mn] - qc);
-            else if (r.end > 0) s = slope_end(lim, qc - sm.Q[v * PT + mp]);
-            else s = slope_interior(lim, qc - sm.Q[v * PT + mp], sm.Q[v * PT + mn] - qc);
-            const double dqh = 0.5 * s;                       // dq_interp = half * f_limiter(q)
-            sm.L[v * PT + me] = qc + dqh;                     // left state of the right face
-            sm.R[v * PT + me] = qc - dqh;                     // right state of the left face
+            for (int v = 0; v < NV; ++v) {
+                const double qc = q[v];
+                double rr = qc;                               // pencil ends: ql(1) = q(1), qr(n-1) = q(n)
+                if (r.end == 0) weno3_faces(Q[v * S + mp], qc, Q[v * S + mn], pp.w_epsilon, q[v], rr);
+                R[v * S + me] = rr;
+            }
+        } else {
+            // an end cell reads its one neighbour on both sides (limited_faces then takes the one difference)
+            const int ap = r.end < 0 ? mn : mp, an = r.end > 0 ? mp : mn;
+            limited_faces<S, 0, PH::NVF>(pp.lim, Q, R, me, ap, an, r.end, q);
+            if constexpr (PH::MHD) limited_faces<S, PH::NVF, NV>(pp.limb, Q, R, me, ap, an, r.end, q);
+        }
+        if constexpr (!KEEP) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) F[v * S + me] = q[v];
         }
     }
     __syncthreads();
     if (r.flux) {
-        if constexpr (FAST) riemann_tile_fast<PH>(sm.L, sm.R, sm.Q, PT, me, mn - me, ch, rcp_nr(ch), pp);
-        else riemann_tile<PH>(sm.L, sm.R, sm.Q, PT, me, mn - me, ch, pp);
+        riemann_cell<PH, S, KEEP, FAST>(q, R + mn, F + me, ch, pp);
+        if constexpr (FC) {
+            if (fc_in) {
+#pragma unroll
+                for (int v = 0; v < NV; ++v) {
+                    const double f = __ldcg(fc_in + v);
+                    F[v * S + me] = f;
+                    if constexpr (KEEP) q[v] = f;
+                }
+            }
+            if (fc_out) {
+#pragma unroll
+                for (int v = 0; v < NV; ++v) fc_out[v] = KEEP ? q[v] : F[v * S + me];
+            }
+        }
+    }
+    if constexpr (FLUX) {
+        if (r.flux) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) w[v] = KEEP ? q[v] : F[v * S + me];
+        }
+        return;
     }
     __syncthreads();
-    if constexpr (FC) {
-        if (r.flux && fc_in) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) sm.Q[v * PT + me] = __ldcg(fc_in + v);
-        }
-        if (r.flux && fc_out) {
-#pragma unroll
-            for (int v = 0; v < NV; ++v) fc_out[v] = sm.Q[v * PT + me];
-        }
-        __syncthreads();
-    }
     if (r.upd) {
         double u0[NV];
         if constexpr (U0S) {
@@ -195,7 +249,7 @@ PK_DEV void rk_stage(const Smem& sm, int me, int mp, int mn, const Roles& r, dou
             load_cell<PH>(u0src, off, g, u0);
         }
 #pragma unroll
-        for (int v = 0; v < NV; ++v) w[v] = u0[v] + dtodx * (sm.Q[v * PT + mp] - sm.Q[v * PT + me]);
+        for (int v = 0; v < NV; ++v) w[v] = u0[v] + dtodx * (F[v * S + mp] - (KEEP ? q[v] : F[v * S + me]));
     } else if (r.keep) {
         load_cell<PH>(wsrc, off, g, w);
     }
@@ -203,7 +257,6 @@ PK_DEV void rk_stage(const Smem& sm, int me, int mp, int mn, const Roles& r, dou
         if constexpr (REC) floors_rec<PH>(w, pp, status, *rec);
         else sources_and_floors<PH>(w, pp, status);
     }
-    __syncthreads();
 }
 
 PK_DEV void flush_status(unsigned status, unsigned* gstatus)
@@ -240,7 +293,7 @@ PK_DEV unsigned short pack_floors(const FloorRec& r1, const FloorRec& r2)
 // (or is the whole pencil, Tile::circ).  REC: also store the stage-1 state of
 // the owned cells in ustar and their floor records in flags (the backward
 // pass's recomputation).
-template <class PH, bool REC = false, bool W3 = false, bool FAST = false>
+template <class PH, int S, bool REC = false, bool W3 = false, bool FAST = false>
 PK_DEV void fused_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, const double* uin, double* uout,
                        const PhysParams& pp, const StepParams* __restrict__ sp, double dl, int apply_fac,
                        double* smem, unsigned& status, double* ustar = nullptr, unsigned short* flags = nullptr)
@@ -252,7 +305,6 @@ PK_DEV void fused_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
     const double ch = stp.ch, psi_fac = apply_fac ? stp.psi_fac : 1.0;
     constexpr int NV = PH::NV;
     const int P = tl.P, T = tl.T, PT = P * T;
-    const Smem sm{smem, smem + NV * PT, smem + 2 * NV * PT, PT};
     const int tid = threadIdx.x;
     int p, t;
     if (tl.xfast) { t = tid % T; p = tid / T; }
@@ -288,7 +340,7 @@ PK_DEV void fused_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
         r.flux = active && (circ || (t >= a + 1 && t < T - a - 2));
         r.upd = active && (circ || (t >= a + 2 && t < T - a - 2));
         FloorRec rec{0, 0};
-        rk_stage<PH, REC, W3, false, FAST>(sm, me, mp, mn, r, w, uin, uin, off, g, stage == 0 ? dtodx1 : dtodx2, ch,
+        rk_stage<PH, S, REC, W3, false, FAST>(smem, me, mp, mn, r, w, uin, uin, off, g, stage == 0 ? dtodx1 : dtodx2, ch,
                                            pp, status, &rec);
         if (stage == 0) {
             rec1 = rec;
@@ -316,7 +368,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sweep_fused(Geom g, Tile tl, con
 {
     extern __shared__ double smem[];
     unsigned status = 0;
-    fused_tile<PH, false, W3, FAST>(g, tl, blockIdx.x * tl.P, blockIdx.y * tl.L, blockIdx.z, uin, uout, pp, sp, dl, apply_fac,
+    fused_tile<PH, MAXT, false, W3, FAST>(g, tl, blockIdx.x * tl.P, blockIdx.y * tl.L, blockIdx.z, uin, uout, pp, sp, dl, apply_fac,
                               smem, status);
     flush_status(status, gstatus);
 }
@@ -387,7 +439,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sweep_batched(const BlockDesc* _
         tl.halo = 4;
         tl.wrap = b.wrap;
         tl.circ = w.circ;
-        fused_tile<PH, false, W3, FAST>(g, tl, w.i1_0, w.c0, w.i2, b.in, b.out, pp, sp, b.dl[dir], apply_fac, smem,
+        fused_tile<PH, MAXT, false, W3, FAST>(g, tl, w.i1_0, w.c0, w.i2, b.in, b.out, pp, sp, b.dl[dir], apply_fac, smem,
                                         status);
     }
     flush_status(status, gstatus);
@@ -443,14 +495,13 @@ PK_DEV void fc_slots(const FcArgs& fc, const Geom& g, int i1, int i2, int s, con
     }
 }
 
-template <class PH, bool W3, bool FC>
+template <class PH, int S, bool W3, bool FC>
 PK_DEV void stage_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, const double* uin, double* uout,
                        double* uh, const PhysParams& pp, int first, double dtodx, double ch, const FcArgs& fc,
                        double* smem, unsigned& status, bool trim = false, bool flat = false)
 {
     constexpr int NV = PH::NV;
     const int P = tl.P, T = tl.T, PT = P * T;
-    const Smem sm{smem, smem + NV * PT, smem + 2 * NV * PT, PT};
     const int tid = threadIdx.x;
     int p, t;
     if (tl.xfast) { t = tid % T; p = tid / T; }
@@ -492,7 +543,7 @@ PK_DEV void stage_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
     double* fc_out = nullptr;
     if constexpr (FC)
         if (valid) fc_slots<PH>(fc, g, i1, i2, s, fc_in, fc_out);
-    rk_stage<PH, false, W3, FC>(sm, me, me - st, me + st, r, w, first ? uin : uh, uin, off, g, dtodx, ch, pp, status,
+    rk_stage<PH, S, false, W3, FC>(smem, me, me - st, me + st, r, w, first ? uin : uh, uin, off, g, dtodx, ch, pp, status,
                                 nullptr, fc_in, fc_out);
     if (own && (!trim || inner)) store_cell<PH>(uout, off, g, w);
 }
@@ -508,7 +559,7 @@ __global__ void __launch_bounds__(MAXT) k_stage(Geom g, Tile tl, const double* u
     extern __shared__ double smem[];
     unsigned status = 0;
     const double dtodx = (rk * spar->dt) / dl;                 // rk_coef(istep) * dt / cg%dl(ddim)
-    stage_tile<PH, W3, FC>(g, tl, blockIdx.x * tl.P, blockIdx.y * tl.L, blockIdx.z, uin, uout, uh, pp, first, dtodx,
+    stage_tile<PH, MAXT, W3, FC>(g, tl, blockIdx.x * tl.P, blockIdx.y * tl.L, blockIdx.z, uin, uout, uh, pp, first, dtodx,
                            spar->ch, fc, smem, status);
     flush_status(status, gstatus);
 }
@@ -557,7 +608,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_stage_batched(const BlockDesc* _
     const double dtodx = (rk * spar->dt) / b.dl[dir];
     const FcArgs fc = fcs ? fcs[w.block] : FcArgs{};
     double* u = const_cast<double*>(b.in);
-    stage_tile<PH, W3, FC>(g, tl, w.i1_0, b.g[dir] - 2, w.i2, u, u, b.uh, pp, first, dtodx, spar->ch, fc, smem, status,
+    stage_tile<PH, MAXT, W3, FC>(g, tl, w.i1_0, b.g[dir] - 2, w.i2, u, u, b.uh, pp, first, dtodx, spar->ch, fc, smem, status,
                            true, true);
     flush_status(status, gstatus);
 }
@@ -672,7 +723,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_stage_refined(const BlockDesc* _
             const double dtodx = (rk * spar->dt) / b.dl[dir];
             const FcArgs fc = fcs ? fcs[it.block] : FcArgs{};
             double* u = const_cast<double*>(b.in);
-            stage_tile<PH, W3, true>(g, tl, it.i1_0, b.g[dir] - 2, 0, u, u, b.uh, pp, first, dtodx, spar->ch, fc,
+            stage_tile<PH, MAXT, W3, true>(g, tl, it.i1_0, b.g[dir] - 2, 0, u, u, b.uh, pp, first, dtodx, spar->ch, fc,
                                      smem, status, true, true);
         } else {
             const long long n = (long long)(it.end - it.beg) * NV;
@@ -713,7 +764,6 @@ __global__ void __launch_bounds__(MAXT, 2) k_unsplit_flux(Geom g, Tile tl, const
     extern __shared__ double smem[];
     constexpr int NV = PH::NV;
     const int P = tl.P, T = tl.T, PT = P * T;
-    const Smem sm{smem, smem + NV * PT, smem + 2 * NV * PT, PT};
     const int tid = threadIdx.x;
     int p, t;
     if (tl.xfast) { t = tid % T; p = tid / T; }
@@ -745,14 +795,9 @@ __global__ void __launch_bounds__(MAXT, 2) k_unsplit_flux(Geom g, Tile tl, const
     double* fc_out = nullptr;
     if constexpr (FC)
         if (valid) fc_slots<PH>(fc, g, i1, i2, s, fc_in, fc_out);
-    rk_stage<PH, false, W3, FC>(sm, me, me - st, me + st, r, w, uin, uin, off, g, 0.0, spar->ch, pp, status, nullptr,
-                                fc_in, fc_out);
-    if (own && r.flux) {
-        double f[NV];
-#pragma unroll
-        for (int v = 0; v < NV; ++v) f[v] = sm.Q[v * PT + me];
-        store_cell<PH>(F, off + g.sd, g, f);
-    }
+    rk_stage<PH, MAXT, false, W3, FC, false, false, true>(smem, me, me - st, me + st, r, w, uin, uin, off, g, 0.0,
+                                                          spar->ch, pp, status, nullptr, fc_in, fc_out);
+    if (own && r.flux) store_cell<PH>(F, off + g.sd, g, w);
 }
 
 }  // namespace pk

@@ -53,6 +53,17 @@ BatchedFn<PH> batched_variant(int v, bool w3 = false)
     }
 }
 
+// the TMA-staged kernel for pencils of n cells (staged_stride)
+template <class PH, bool FAST = false, bool REC = false>
+auto staged_kernel(int n) -> decltype(&k_sweep_staged<PH, 256, FAST, REC>)
+{
+    switch (staged_stride(n)) {
+    case 64: return k_sweep_staged<PH, 64, FAST, REC>;
+    case 128: return k_sweep_staged<PH, 128, FAST, REC>;
+    default: return k_sweep_staged<PH, 256, FAST, REC>;
+    }
+}
+
 // dynamic shared memory limits of the fused and batched sweep kernels
 template <class PH, bool FAST>
 int set_fused_attr(pk_ctx* h)
@@ -69,8 +80,9 @@ int set_fused_attr(pk_ctx* h)
                                         220 * 1024));
         PK_CUDA(h, cudaFuncSetAttribute(batched_variant<PH, FAST>(0, true),
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-        PK_CUDA(h, cudaFuncSetAttribute(k_sweep_staged<PH, FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        220 * 1024));
+        for (int n : {64, 128, 256})
+            PK_CUDA(h, cudaFuncSetAttribute(staged_kernel<PH, FAST>(n), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            220 * 1024));
         done = true;
     }
     return PK_OK;
@@ -203,10 +215,10 @@ int launch_fused_ptr(pk_ctx* h, Block& b, int dir, int apply_fac, const double* 
             return fail(h, PK_E_CUDA, "cuTensorMapEncodeTiled failed for the staged sweep");
         const int threads = (b.n[dir] + 31) / 32 * 32;
         if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
-        k_sweep_staged<PH, FAST><<<grid, threads, staged_smem(PH::NV, b.n[dir]), h->stream>>>(
+        staged_kernel<PH, FAST>(b.n[dir])<<<grid, threads, staged_smem(PH::NV, b.n[dir]), h->stream>>>(
             tin, tout, g, h->pp, b.dl[dir], h->d_step, apply_fac, dir, h->d_status, nullptr, nullptr);
     } else {
-        const size_t smem = 3ull * PH::NV * tl.P * tl.T * sizeof(double);
+        const size_t smem = 3ull * PH::NV * VAR_T[var] * sizeof(double);
         if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
         fused_variant<PH, FAST>(var, h->pp.weno3)<<<grid, tl.P * tl.T, smem, h->stream>>>(g, tl, in, out, h->pp,
                                                                                          b.dl[dir], h->d_step,
@@ -260,8 +272,9 @@ int launch_fused_rec(pk_ctx* h, Block& b, int dir, int apply_fac, const double* 
             for (int v = 0; v < NVARIANT; ++v)
                 PK_CUDA(h, cudaFuncSetAttribute(rec_variant<PH>(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                 220 * 1024));
-            PK_CUDA(h, cudaFuncSetAttribute(k_sweep_staged<PH, false, true>,
-                                            cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+            for (int n : {64, 128, 256})
+                PK_CUDA(h, cudaFuncSetAttribute(staged_kernel<PH, false, true>(n),
+                                                cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
             attr = true;
         }
         Geom g = make_geom(b, dir);
@@ -277,10 +290,10 @@ int launch_fused_rec(pk_ctx* h, Block& b, int dir, int apply_fac, const double* 
                 return fail(h, PK_E_CUDA, "cuTensorMapEncodeTiled failed for the staged sweep");
             const int threads = (b.n[dir] + 31) / 32 * 32;
             if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
-            k_sweep_staged<PH, false, true><<<grid, threads, staged_smem(PH::NV, b.n[dir]), h->stream>>>(
+            staged_kernel<PH, false, true>(b.n[dir])<<<grid, threads, staged_smem(PH::NV, b.n[dir]), h->stream>>>(
                 tin, tout, g, h->pp, b.dl[dir], h->d_step, apply_fac, dir, h->d_status, ustar, flags);
         } else {
-            const size_t smem = 3ull * PH::NV * tl.P * tl.T * sizeof(double);
+            const size_t smem = 3ull * PH::NV * VAR_T[var] * sizeof(double);
             if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
             rec_variant<PH>(var)<<<grid, tl.P * tl.T, smem, h->stream>>>(g, tl, in, out, ustar, flags, h->pp,
                                                                         b.dl[dir], h->d_step, apply_fac, h->d_status);
@@ -495,7 +508,7 @@ int launch_stage(pk_ctx* h, Block& b, int dir, int first, double rk)
     }
     tl.xfast = (dir == 0);
     dim3 grid((g.n1 + tl.P - 1) / tl.P, (ext + tl.L - 1) / tl.L, g.n2);
-    const size_t smem = 3ull * PH::NV * tl.P * tl.T * sizeof(double);
+    const size_t smem = 3ull * PH::NV * STAGE_MAXT * sizeof(double);
     std::pair<cudaEvent_t, cudaEvent_t> ev;
     if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
     const FcArgs& fc = b.fc[dir];
@@ -607,7 +620,7 @@ int launch_unsplit_flux(pk_ctx* h, Block& b, int dir, const double* in, double* 
     }
     tl.xfast = (dir == 0);
     dim3 grid((g.n1 + tl.P - 1) / tl.P, (ext + tl.L - 1) / tl.L, g.n2);
-    const size_t smem = 3ull * PH::NV * tl.P * tl.T * sizeof(double);
+    const size_t smem = 3ull * PH::NV * UNSPLIT_MAXT * sizeof(double);
     std::pair<cudaEvent_t, cudaEvent_t> ev;
     if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
     // a refined block's fine/coarse flux couplings along dir (ext_fluxes, unsplit_mag_modules.F90:195-204)

@@ -21,8 +21,9 @@
 // each CTA taking its instance's step scalars), n <= 256 along
 // the sweep, an even x extent and an even x guard width (the box's x
 // coordinate and the tensor strides must be multiples of 16 bytes), linear
-// reconstruction.  Shared memory: 2n planes-worth of doubles for the box plus
-// the three n-cell planes of the tile per component.
+// reconstruction.  Shared memory: 2n doubles per component for the box plus the
+// tile's three planes of S doubles, S the smallest of 64, 128 and 256 that
+// holds the pencil (a kernel of its own each: S is the launch bound too).
 //
 // REC (the backward pass's recomputation, bit-exact arithmetic only): also
 // store each cell's stage-1 state in ustar and its floor records in flags, as
@@ -88,8 +89,8 @@ PK_DEV void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" 
 // ---------------------------------------------------------------------------
 // grid: x = pairs of pencils along ortho-1, y = 1, z = ortho-2; blockDim.x >= n
 // ---------------------------------------------------------------------------
-template <class PH, bool FAST = false, bool REC = false>
-__global__ void __launch_bounds__(256, 2) k_sweep_staged(const __grid_constant__ CUtensorMap tin,
+template <class PH, int S, bool FAST = false, bool REC = false>
+__global__ void __launch_bounds__(S, 512 / S) k_sweep_staged(const __grid_constant__ CUtensorMap tin,
                                                          const __grid_constant__ CUtensorMap tout, Geom g,
                                                          PhysParams pp, double dl, const StepParams* __restrict__ sp,
                                                          int apply_fac, int dir, unsigned* __restrict__ gstatus,
@@ -100,8 +101,8 @@ __global__ void __launch_bounds__(256, 2) k_sweep_staged(const __grid_constant__
     extern __shared__ __align__(128) double smem[];
     const int n = g.n_d;
     double* box = smem;                                  // [NV][2n] in the box's element order
-    const Smem sm{box + 2 * NV * n, box + 3 * NV * n, box + 4 * NV * n, n};
-    unsigned long long* bar = reinterpret_cast<unsigned long long*>(box + 5 * NV * n);
+    double* sm = box + 2 * NV * n;                       // the tile's planes
+    unsigned long long* bar = reinterpret_cast<unsigned long long*>(sm + tile_doubles<PH, S>());
     // element strides of the box along the pencil (t) and across the pair (p)
     const int st_t = dir == 0 ? 1 : 2, st_p = dir == 0 ? n : 1;
     const int i1_0 = 2 * blockIdx.x, i2 = blockIdx.z;
@@ -158,7 +159,7 @@ __global__ void __launch_bounds__(256, 2) k_sweep_staged(const __grid_constant__
 #pragma unroll 1
         for (int s = 0; s < 2; ++s) {
             FloorRec rec{0, 0};
-            rk_stage<PH, REC, false, false, FAST, true>(sm, t, mp, mn, r, w, nullptr, nullptr, 0, g,
+            rk_stage<PH, S, REC, false, false, FAST, true>(sm, t, mp, mn, r, w, nullptr, nullptr, 0, g,
                                                         s == 0 ? dtodx1 : dtodx2, ch, pp, status, &rec, nullptr,
                                                         nullptr, mine, 2 * n);
             if constexpr (REC) {
@@ -235,7 +236,14 @@ inline bool encode_state_map(CUtensorMap* m, const double* base, const int n[3],
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// dynamic shared memory of a staged tile of nv planes and n cells (+ the mbarrier)
-inline size_t staged_smem(int nv, int n) { return (size_t)5 * nv * n * sizeof(double) + 16; }
+// the shared planes' stride (and launch bound) of a staged tile of n cells
+inline int staged_stride(int n) { return n <= 64 ? 64 : (n <= 128 ? 128 : 256); }
+
+// dynamic shared memory of a staged tile of nv planes and n cells: the box, the
+// tile's planes and the mbarrier
+inline size_t staged_smem(int nv, int n)
+{
+    return ((size_t)2 * nv * n + (size_t)3 * nv * staged_stride(n)) * sizeof(double) + 16;
+}
 
 }  // namespace pk
