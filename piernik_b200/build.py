@@ -22,7 +22,7 @@ FAST_UNITS = [f"pk_fast_{p}.cu" for p in PHYS]
 UNITS = (["pk_api.cu", "pk_noalloc.cu", "pk_peak.cu", "pk_exchange.cpp", "pk_levels.cpp"]
          + [f"pk_phys_{p}.cu" for p in PHYS] + FAST_UNITS)
 HEADERS = ["pk_device.cuh", "pk_kernels.cuh", "pk_aux.cuh", "pk_internal.h", "pk_launch.cuh", "pk_adjoint.cuh", "pk_levels.h",
-           "pk_adjoint_kernels.cuh", "pk_exchange.h", "pk_fast.cuh", "pk_staged.cuh"]
+           "pk_adjoint_kernels.cuh", "pk_exchange.h", "pk_fast.cuh", "pk_staged.cuh", "pk_quotient.cuh"]
 DEPS = [os.path.join(CSRC, f) for f in UNITS + HEADERS]
 INC = os.path.join(os.path.dirname(HERE), "include")
 OUT = os.path.join(HERE, "libpiernik_b200.so")

@@ -853,6 +853,7 @@ int put_step_params(pk_ctx* h, double dt, double ch, double fac)
         h->h_step[i].dt = dt;
         h->h_step[i].ch = ch;
         h->h_step[i].psi_fac = fac;
+        h->h_step[i].rch = 1.0 / ch;
     }
     PK_CUDA(h, cudaMemcpyAsync(h->d_step, h->h_step, sizeof(StepParams) * h->ninst, cudaMemcpyHostToDevice, h->stream));
     return PK_OK;
@@ -866,6 +867,7 @@ int put_step_array(pk_ctx* h, const StepRec* r)
         h->h_step[i].dt = r[i].dt;
         h->h_step[i].ch = r[i].ch;
         h->h_step[i].psi_fac = r[i].fac;
+        h->h_step[i].rch = 1.0 / r[i].ch;
     }
     PK_CUDA(h, cudaMemcpyAsync(h->d_step, h->h_step, sizeof(StepParams) * h->ninst, cudaMemcpyHostToDevice, h->stream));
     return PK_OK;

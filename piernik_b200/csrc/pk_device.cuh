@@ -107,22 +107,40 @@ enum StatusBits : unsigned {
     ST_EI_NEGATIVE = 2u,   // ei_negative (sources.F90:422)
 };
 
+// The arithmetic of utoq and of the Riemann solves, passed as a policy (Ieee
+// here; Exact, the kernels', in pk_quotient.cuh; Fast, the tolerance mode's, in
+// pk_fast.cuh).  inv(d) is taken once per denominator and used by every
+// quo(n, d, inv(d)); quoz is quo for numerators that are often exactly zero;
+// quoc divides by a constant d whose correctly rounded reciprocal y is known;
+// root(x, aux) is sqrt(x), and over_root(n, root, aux) is n / that root.  ok()
+// tells whether all quotients taken so far are the correctly rounded ones.
+struct Ieee {
+    static constexpr bool FAST = false;
+    PK_PHYS double inv(double) { return 0.0; }
+    PK_PHYS double quo(double n, double d, double) { return n / d; }
+    PK_PHYS double quoz(double n, double d, double) { return n / d; }
+    PK_PHYS double quoc(double n, double d, double) { return n / d; }
+    PK_PHYS double root(double x, double&) { return sqrt(x); }
+    PK_PHYS double over_root(double n, double root, double) { return n / root; }
+    PK_PHYS bool ok() const { return true; }
+};
+
 // -------------------------------------------------------------------------
 // utoq: conservative -> primitive, one cell (interpolations.F90:69-106)
 // -------------------------------------------------------------------------
-template <class PH>
-PK_PHYS void utoq(const double (&u)[PH::NV], double (&q)[PH::NV], const PhysParams& pp)
+template <class PH, class A>
+PK_PHYS void utoq(A& ar, const double (&u)[PH::NV], double (&q)[PH::NV], const PhysParams& pp)
 {
 #pragma unroll
     for (int f = 0; f < PH::NFL; ++f) {
         const int b = PH::beg(f);
-        const double dn = u[b], mx = u[b + 1], my = u[b + 2], mz = u[b + 3];
+        const double dn = u[b], mx = u[b + 1], my = u[b + 2], mz = u[b + 3], r = ar.inv(dn);
         q[b] = dn;
-        q[b + 1] = mx / dn;
-        q[b + 2] = my / dn;
-        q[b + 3] = mz / dn;
+        q[b + 1] = ar.quoz(mx, dn, r);
+        q[b + 2] = ar.quoz(my, dn, r);
+        q[b + 3] = ar.quoz(mz, dn, r);
         if (PH::has_en(f)) {
-            const double ek = (0.5 * ((mx * mx + my * my) + mz * mz)) / dn;
+            const double ek = ar.quoz(0.5 * ((mx * mx + my * my) + mz * mz), dn, r);
             double p = pp.gam_1[f] * (u[b + 4] - ek);
             if (PH::magn(f)) {
                 const double bx = u[PH::IB], by = u[PH::IB + 1], bz = u[PH::IB + 2];
@@ -135,6 +153,13 @@ PK_PHYS void utoq(const double (&u)[PH::NV], double (&q)[PH::NV], const PhysPara
 #pragma unroll
         for (int c = 0; c < 4; ++c) q[PH::IB + c] = u[PH::IB + c];   // B and psi go to blimiter as they are
     }
+}
+
+template <class PH>
+PK_PHYS void utoq(const double (&u)[PH::NV], double (&q)[PH::NV], const PhysParams& pp)
+{
+    Ieee ar;
+    utoq<PH>(ar, u, q, pp);
 }
 
 // -------------------------------------------------------------------------
@@ -214,328 +239,307 @@ PK_PHYS double slope_end(int lim, double d)
 // bf: transverse B fluxes.
 // -------------------------------------------------------------------------
 
-// Physical flux of one side (hlld.F90:296-308): fluid part f[0..nc) and the
-// transverse B fluxes bf[1..2].  Computed where needed so that neither side's
-// flux is held in registers through the star-state algebra.
-PK_PHYS void side_flux(bool has_energy, const double* u, const double* b, double pr, double en, double* f)
-{
-    f[0] = u[0] * u[1];
-    f[1] = ((u[0] * (u[1] * u[1])) + pr) - (b[0] * b[0]);
-    f[2] = ((u[0] * u[2]) * u[1]) - (b[0] * b[1]);
-    f[3] = ((u[0] * u[3]) * u[1]) - (b[0] * b[2]);
-    if (has_energy) f[4] = ((en + pr) * u[1]) - (b[0] * ((u[1] * b[0] + u[2] * b[1]) + u[3] * b[2]));
-}
-
+// transverse B flux of one side (b_cclf(ydim:zdim), hlld.F90:301,309)
 PK_PHYS double side_bflux(const double* u, const double* b, int c)
 {
-    return (b[c] * u[1]) - (b[0] * u[1 + c]);     // b_cclf(ydim:zdim), hlld.F90:301,309
+    return (b[c] * u[1]) - (b[0] * u[1 + c]);
 }
 
-// [ u(idn), u(idn)*u(imx:imz), en ] of one side
-PK_PHYS double side_cons(const double* u, double en, int c)
+// HLLD flux of one interface (riemann_hlld, hlld.F90:161-609).  Everything up to
+// the Alfven speeds is computed for both sides, whose chains of dependent
+// quotients and roots overlap; then the side that the flux is taken from (both
+// where sm = 0) is picked by selects, and its energy, its star energy and its
+// flux are computed for that side only.
+template <class A>
+PK_PHYS void hlld_face(A& ar, bool has_energy, double gamma, double rgam_1, double rgam, const double (&ul)[5],
+                       const double (&ur)[5], const double (&bl)[3], const double (&br)[3], double (&f)[5],
+                       double (&bf)[2])
 {
-    return c == 0 ? u[0] : (c == 4 ? en : u[0] * u[c]);
+    const bool dust = gamma < 0.0;
+    const double bbl = (bl[0] * bl[0] + bl[1] * bl[1]) + bl[2] * bl[2];
+    const double bbr = (br[0] * br[0] + br[1] * br[1]) + br[2] * br[2];
+    double prl = 0.0, prr = 0.0, c_fastm = 0.0;                                      // hlld.F90:245-249
+    if (!dust) {
+        prl = ul[4] + 0.5 * bbl;                                                      // :239-240, 258-259
+        prr = ur[4] + 0.5 * bbr;
+        const double gampr_l = gamma * ul[4];
+        const double gampr_r = gamma * ur[4];
+        const double al = gampr_l + bbl, ar_ = gampr_r + bbr;                        // :272-274
+        const double nl = al + sqrt(al * al - ((4.0 * gampr_l) * (bl[0] * bl[0])));
+        const double nr = ar_ + sqrt(ar_ * ar_ - ((4.0 * gampr_r) * (br[0] * br[0])));
+        double cmax;
+        if constexpr (A::FAST) {               // max(nl/rho_l, nr/rho_r) with one quotient (densities are positive)
+            const bool lm = nl * ur[0] >= nr * ul[0];
+            cmax = ar.div(lm ? nl : nr, lm ? ul[0] : ur[0]);
+        } else {
+            cmax = f_max(ar.quo(nl, ul[0], ar.inv(ul[0])), ar.quo(nr, ur[0], ar.inv(ur[0])));
+        }
+        c_fastm = sqrt(0.5 * cmax);
+    }
+    const double sl = f_min(ul[1], ur[1]) - c_fastm;                                // :291-292
+    const double sr = f_max(ul[1], ur[1]) + c_fastm;
+
+    // the flux of the picked side, from its energy on: fs alone (FAN 0, :312-319),
+    // fs + s (u* - u) (FAN 1, Eq. 64), or ((fs + a u**) - (a - s) u*) - s u (FAN 2,
+    // Eq. 65); add: the second of two sides whose mean is the flux
+    double sm = 0.0, prt_star = 0.0, us0 = 0.0, vs[2] = {0.0, 0.0}, bs[2] = {0.0, 0.0}, a = 0.0, root = 0.0;
+    double v2[2] = {0.0, 0.0}, b2[2] = {0.0, 0.0}, b2n = 0.0, rssm = 0.0;
+    auto side = [&](bool left, int fan, bool add) {
+        double u[5], b[3];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) u[c] = left ? ul[c] : ur[c];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) b[c] = left ? bl[c] : br[c];
+        const double s = left ? sl : sr, pr = left ? prl : prr;
+        double en = 1.7976931348623157e308;
+        if (!dust) {                                                                 // :260-269
+            double ei;
+            if constexpr (A::FAST) ei = u[4] * rgam_1;
+            else ei = ar.quoc(u[4], gamma - 1.0, rgam_1);
+            en = (ei + ((0.5 * u[0]) * ((u[1] * u[1] + u[2] * u[2]) + u[3] * u[3]))) + (0.5 * (left ? bbl : bbr));
+        }
+        const double vb = (u[1] * b[0] + u[2] * b[1]) + u[3] * b[2];
+        double us4 = 0.0, u24 = 0.0;
+        if (fan && has_energy) {                                                     // :388-404
+            const double vb_star = (sm * b[0] + vs[0] * bs[0]) + vs[1] * bs[1];
+            us4 = ar.quo(((((s - u[1]) * en) - (pr * u[1])) + (prt_star * sm)) + (b[0] * (vb - vb_star)), s - sm, rssm);
+            if (fan == 2) {                                                          // :474-489
+                const double vb_2star = (sm * b2n + v2[0] * b2[0]) + v2[1] * b2[1];
+                const double t = (((bl[0] >= 0.0) ? 1.0 : -1.0) * root) * (vb_star - vb_2star);
+                u24 = left ? us4 - t : us4 + t;
+            }
+        }
+        // side_flux (:296-309), the conserved state, u* and u**
+        const double uc[7] = {u[0], u[0] * u[1], u[0] * u[2], u[0] * u[3], en, b[1], b[2]};
+        const double fs[7] = {uc[1], ((u[0] * (u[1] * u[1])) + pr) - (b[0] * b[0]), (uc[2] * u[1]) - (b[0] * b[1]),
+                              (uc[3] * u[1]) - (b[0] * b[2]), ((en + pr) * u[1]) - (b[0] * vb),
+                              (b[1] * u[1]) - (b[0] * u[2]), (b[2] * u[1]) - (b[0] * u[3])};
+        const double us[7] = {us0, us0 * sm, us0 * vs[0], us0 * vs[1], us4, bs[0], bs[1]};
+        const double u2[7] = {us0, us0 * sm, us0 * v2[0], us0 * v2[1], u24, b2[0], b2[1]};
+        const double ams = a - s;
+#pragma unroll
+        for (int c = 0; c < 7; ++c) {
+            double o = fs[c];
+            const double p = c < 5 ? f[c] : bf[c - 5];
+            if (fan == 2) {
+                o = ((fs[c] + a * u2[c]) - ams * us[c]) - s * uc[c];
+                if (add) o = 0.5 * (p + o);                                          // :524-544
+            } else if (fan == 1) {
+                const double d = s * (us[c] - uc[c]);
+                o = add ? 0.5 * ((p + fs[c]) + d) : fs[c] + d;                       // :583-599, summed left to right
+            }
+            if (c < 5) f[c] = o;
+            else bf[c - 5] = o;
+        }
+    };
+
+    if (sl >= 0.0 || sr <= 0.0) {                                                    // :312-319
+        side(sl >= 0.0, 0, false);
+        return;
+    }
+    const double slvxl = sl - ul[1], srvxr = sr - ur[1];                            // :323-330, 344-347
+    const double dn_l = ul[0] * slvxl, dn_r = ur[0] * srvxr;
+    {
+        const double n = (dn_r * ur[1] - prr) - (dn_l * ul[1] - prl), d = dn_r - dn_l;
+        if (fabs(d) < f_spacing(dn_r + dn_l)) {
+            sm = (sl + sr) * 0.5;
+        } else {
+            if constexpr (A::FAST) sm = ar.div(n, d);
+            else sm = ar.quoz(n, d, ar.inv(d));
+        }
+    }
+    const double slsm = sl - sm, srsm = sr - sm;                                    // :334-340
+    const double b_lr = bl[0] * br[0];
+    double b_lrgam;
+    if constexpr (A::FAST) b_lrgam = b_lr * rgam;
+    else b_lrgam = ar.quoc(b_lr, gamma, rgam);
+    prt_star = 0.5 * ((prl + dn_l * (sm - ul[1])) + (prr + dn_r * (sm - ur[1])));
+    // rho*, transverse B* (HLL fallback) and v* of both sides (:354-355, :362-382)
+    const double rslsm = ar.inv(slsm), rsrsm = ar.inv(srsm);
+    const double usl0 = ar.quo(dn_l, slsm, rslsm), usr0 = ar.quo(dn_r, srsm, rsrsm);
+    double bsl[2], bsr[2], vsl[2], vsr[2];
+    {
+        const double cl = dn_l * slsm - b_lr, cr = dn_r * srsm - b_lr;
+        const bool star_l = (fabs(cl) > f_spacing(b_lr)) && b_lrgam <= (has_energy ? ul[4] : 0.0);
+        const bool star_r = (fabs(cr) > f_spacing(b_lr)) && b_lrgam <= (has_energy ? ur[4] : 0.0);
+        const double tl = dn_l * slvxl - b_lr, tr = dn_r * srvxr - b_lr;
+        if constexpr (A::FAST) {
+            const double ql = ar.div(tl, cl), qr = ar.div(tr, cr);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                bsl[c] = bl[1 + c] * ql;
+                bsr[c] = br[1 + c] * qr;
+            }
+        } else {
+            const double dl = star_l ? cl : 1.0, dr = star_r ? cr : 1.0;
+            const double rl = ar.inv(dl), rr = ar.inv(dr);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                bsl[c] = ar.quoz(bl[1 + c] * tl, dl, rl);
+                bsr[c] = ar.quoz(br[1 + c] * tr, dr, rr);
+            }
+        }
+        if (!(star_l && star_r)) {
+            const double d = sr - sl, r = ar.inv(d);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const double h = ar.quoz((sr * br[1 + c] - sl * bl[1 + c]) - (side_bflux(ur, br, 1 + c) - side_bflux(ul, bl, 1 + c)), d, r);
+                if (!star_l) bsl[c] = h;
+                if (!star_r) bsr[c] = h;
+            }
+        }
+        double kl, kr;
+        if constexpr (A::FAST) {
+            kl = ar.div(bl[0], dn_l);
+            kr = ar.div(br[0], dn_r);
+        } else {
+            kl = ar.quoz(bl[0], dn_l, ar.inv(dn_l));
+            kr = ar.quoz(br[0], dn_r, ar.inv(dn_r));
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            vsl[c] = ul[2 + c] + (kl * (bl[1 + c] - bsl[c]));
+            vsr[c] = ur[2 + c] + (kr * (br[1 + c] - bsr[c]));
+        }
+    }
+    bool left = sm > 0.0, both = !left && !(sm < 0.0), alfven = false;
+    double rtl = 0.0, rtr = 0.0, alfven_l = 0.0, alfven_r = 0.0;
+    if (fabs(bl[0]) > 0.0) {                                                         // :410-448
+        double xl = 0.0, xr = 0.0;
+        rtl = ar.root(usl0, xl);
+        rtr = ar.root(usr0, xr);
+        alfven_l = sm - ar.over_root(fabs(bl[0]), rtl, xl);
+        alfven_r = sm + ar.over_root(fabs(br[0]), rtr, xr);
+        alfven = !(alfven_l > 0.0 || alfven_r < 0.0);
+        if (!alfven) {
+            left = alfven_l > 0.0;
+            both = false;
+        } else {                                                                     // :452-470
+            const double b_sig = (bl[0] >= 0.0) ? 1.0 : -1.0;
+            const double d = rtl + rtr, r = ar.inv(d), bsm = b_sig * (rtl * rtr);
+            b2n = 0.5 * (bl[0] + br[0]);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                v2[c] = ar.quoz((rtl * vsl[c] + rtr * vsr[c]) + b_sig * (bsr[c] - bsl[c]), d, r);
+                b2[c] = ar.quoz((rtl * bsr[c] + rtr * bsl[c]) + bsm * (vsr[c] - vsl[c]), d, r);
+            }
+        }
+    }
+    auto pick = [&](bool l) {
+        us0 = l ? usl0 : usr0;
+        rssm = l ? rslsm : rsrsm;
+        root = l ? rtl : rtr;
+        a = l ? alfven_l : alfven_r;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            vs[c] = l ? vsl[c] : vsr[c];
+            bs[c] = l ? bsl[c] : bsr[c];
+        }
+    };
+    left = left || both;
+    pick(left);
+    side(left, alfven ? 2 : 1, false);
+    if (both) {                                                                      // sm = 0
+        pick(false);
+        side(false, alfven ? 2 : 1, true);
+    }
+}
+
+// HLLC flux of one interface (riemann_hlld_u, hlld.F90:615-841): the side the flux
+// is taken from picked by selects, both where sm = 0.
+template <class A>
+PK_PHYS void hllc_face(A& ar, bool has_energy, double gamma, double rgam_1, const double (&ul)[5],
+                       const double (&ur)[5], double (&f)[5])
+{
+    const bool dust = gamma < 0.0;
+    double prl = 0.0, prr = 0.0, c_fastm = 0.0;                                      // hlld.F90:673-677
+    if (!dust) {                                                                     // :689-703
+        prl = ul[4];
+        prr = ur[4];
+        const double gampr_l = gamma * ul[4];
+        const double gampr_r = gamma * ur[4];
+        double cmax;
+        if constexpr (A::FAST) {
+            const bool lm = gampr_l * ur[0] >= gampr_r * ul[0];
+            cmax = ar.div(lm ? gampr_l : gampr_r, lm ? ul[0] : ur[0]);
+        } else {
+            cmax = f_max(ar.quo(gampr_l, ul[0], ar.inv(ul[0])), ar.quo(gampr_r, ur[0], ar.inv(ur[0])));
+        }
+        c_fastm = sqrt(cmax);
+    }
+    const double sl = f_min(ul[1], ur[1]) - c_fastm;                                // :719-720
+    const double sr = f_max(ul[1], ur[1]) + c_fastm;
+    const bool fan = !(sl >= 0.0 || sr <= 0.0);                                      // :738-743
+    bool left = sl >= 0.0, both = false;
+    double sm = 0.0, prt_star = 0.0;
+    if (fan) {
+        const double dn_l = ul[0] * (sl - ul[1]), dn_r = ur[0] * (sr - ur[1]);       // :747-764
+        const double n = (dn_r * ur[1] - prr) - (dn_l * ul[1] - prl), d = dn_r - dn_l;
+        if (fabs(d) < f_spacing(dn_r + dn_l)) {
+            sm = (sl + sr) * 0.5;
+        } else {
+            if constexpr (A::FAST) sm = ar.div(n, d);
+            else sm = ar.quoz(n, d, ar.inv(d));
+        }
+        prt_star = 0.5 * ((prl + dn_l * (sm - ul[1])) + (prr + dn_r * (sm - ur[1])));
+        left = !(sm < 0.0);
+        both = left && !(sm > 0.0);
+    }
+    auto side = [&](bool l, bool add) {
+        double u[5];
+#pragma unroll
+        for (int c = 0; c < 5; ++c) u[c] = l ? ul[c] : ur[c];
+        const double s = l ? sl : sr, pr = l ? prl : prr;
+        double en = 1.7976931348623157e308;
+        if (!dust) {
+            double ei;
+            if constexpr (A::FAST) ei = u[4] * rgam_1;
+            else ei = ar.quoc(u[4], gamma - 1.0, rgam_1);
+            en = ei + ((0.5 * u[0]) * ((u[1] * u[1] + u[2] * u[2]) + u[3] * u[3]));
+        }
+        const double uc[5] = {u[0], u[0] * u[1], u[0] * u[2], u[0] * u[3], en};
+        const double fs[5] = {uc[1], (u[0] * (u[1] * u[1])) + pr, uc[2] * u[1], uc[3] * u[1], (en + pr) * u[1]};   // :724-734
+        if (!fan) {
+#pragma unroll
+            for (int c = 0; c < 5; ++c) f[c] = fs[c];
+            return;
+        }
+        const double svx = s - u[1], ssm = s - sm, rssm = ar.inv(ssm);               // :771-796
+        const double us0 = ar.quo(u[0] * svx, ssm, rssm);
+        double us[5] = {us0, us0 * sm, us0 * u[2], us0 * u[3], 0.0};
+        if (has_energy) us[4] = ar.quo(((svx * en) - (pr * u[1])) + (prt_star * sm), ssm, rssm);
+#pragma unroll
+        for (int c = 0; c < 5; ++c) {                                                // :798-829
+            const double d = s * (us[c] - uc[c]);
+            f[c] = add ? 0.5 * ((f[c] + fs[c]) + d) : fs[c] + d;
+        }
+    };
+    side(left, false);
+    if (both) side(false, true);
 }
 
 PK_PHYS void hlld_iface(bool has_energy, double gamma, const double* ul, const double* ur, const double* bl,
                        const double* br, double* f, double* bf)
 {
-    const int nc = has_energy ? 5 : 4;
-    double prl, prr, c_fastm;
-    double enl = 1.7976931348623157e308, enr = 1.7976931348623157e308, ue = 0.0;
-
-    const double magprl = 0.5 * ((bl[0] * bl[0] + bl[1] * bl[1]) + bl[2] * bl[2]);   // hlld.F90:239-240
-    const double magprr = 0.5 * ((br[0] * br[0] + br[1] * br[1]) + br[2] * br[2]);
-    if (gamma < 0.0) {                                                               // :245-249
-        prl = 0.0;
-        prr = 0.0;
-        c_fastm = 0.0;
-    } else {
-        prl = ul[4] + magprl;                                                         // :258-259
-        prr = ur[4] + magprr;
-        const double bbl = (bl[0] * bl[0] + bl[1] * bl[1]) + bl[2] * bl[2];
-        const double bbr = (br[0] * br[0] + br[1] * br[1]) + br[2] * br[2];
-        enl = ((ul[4] / (gamma - 1.0)) + ((0.5 * ul[0]) * ((ul[1] * ul[1] + ul[2] * ul[2]) + ul[3] * ul[3]))) + (0.5 * bbl);
-        enr = ((ur[4] / (gamma - 1.0)) + ((0.5 * ur[0]) * ((ur[1] * ur[1] + ur[2] * ur[2]) + ur[3] * ur[3]))) + (0.5 * bbr);
-        const double gampr_l = gamma * ul[4];
-        const double gampr_r = gamma * ur[4];
-        const double al = gampr_l + bbl, ar = gampr_r + bbr;                         // :272-274
-        const double cl = (al + sqrt(al * al - ((4.0 * gampr_l) * (bl[0] * bl[0])))) / ul[0];
-        const double cr = (ar + sqrt(ar * ar - ((4.0 * gampr_r) * (br[0] * br[0])))) / ur[0];
-        c_fastm = sqrt(0.5 * f_max(cl, cr));
-    }
-    const double sl = f_min(ul[1], ur[1]) - c_fastm;                                // :291-292
-    const double sr = f_max(ul[1], ur[1]) + c_fastm;
-
-    if (sl >= 0.0 || sr <= 0.0) {                                                    // :312-319
-        const bool left = sl >= 0.0;
-        const double* u = left ? ul : ur;
-        const double* b = left ? bl : br;
-        side_flux(has_energy, u, b, left ? prl : prr, left ? enl : enr, f);
-        bf[0] = side_bflux(u, b, 1);
-        bf[1] = side_bflux(u, b, 2);
-        return;
-    }
-
-    double sm;                                                                       // :323-330
-    {
-        const double auxr = (sr - ur[1]) * ur[0];
-        const double auxl = (sl - ul[1]) * ul[0];
-        if (fabs(auxr - auxl) < f_spacing(auxr + auxl)) sm = (sl + sr) / 2.0;
-        else sm = ((auxr * ur[1] - prr) - (auxl * ul[1] - prl)) / (auxr - auxl);
-    }
-    const double slsm = sl - sm, srsm = sr - sm;                                    // :334-340
-    const double slvxl = sl - ul[1], srvxr = sr - ur[1];
-    const double srmsl = sr - sl;
-    const double dn_l = ul[0] * slvxl, dn_r = ur[0] * srvxr;                        // :344-347
-    const double b_lr = bl[0] * br[0];
-    const double b_lrgam = b_lr / gamma;
-    const double prt_star = 0.5 * ((prl + dn_l * (sm - ul[1])) + (prr + dn_r * (sm - ur[1])));
-
-    // transverse B of the star states, with the HLL fallback (:362-378)
-    double bsl[3], bsr[3];
-    bsl[0] = bl[0];
-    bsr[0] = br[0];
-    {
-        const double bclf1 = side_bflux(ul, bl, 1), bclf2 = side_bflux(ul, bl, 2);
-        const double bcrf1 = side_bflux(ur, br, 1), bcrf2 = side_bflux(ur, br, 2);
-        double coeff_1 = dn_l * slsm - b_lr;
-        if (has_energy) ue = ul[4];
-        if ((fabs(coeff_1) > f_spacing(b_lr)) && b_lrgam <= ue) {
-            const double a = dn_l * slvxl - b_lr;
-            bsl[1] = (bl[1] * a) / coeff_1;
-            bsl[2] = (bl[2] * a) / coeff_1;
-        } else {
-            bsl[1] = ((sr * br[1] - sl * bl[1]) - (bcrf1 - bclf1)) / srmsl;
-            bsl[2] = ((sr * br[2] - sl * bl[2]) - (bcrf2 - bclf2)) / srmsl;
-        }
-        coeff_1 = dn_r * srsm - b_lr;
-        if (has_energy) ue = ur[4];
-        if ((fabs(coeff_1) > f_spacing(b_lr)) && b_lrgam <= ue) {
-            const double a = dn_r * srvxr - b_lr;
-            bsr[1] = (br[1] * a) / coeff_1;
-            bsr[2] = (br[2] * a) / coeff_1;
-        } else {
-            bsr[1] = ((sr * br[1] - sl * bl[1]) - (bcrf1 - bclf1)) / srmsl;
-            bsr[2] = ((sr * br[2] - sl * bl[2]) - (bcrf2 - bclf2)) / srmsl;
-        }
-    }
-    double vsl[3], vsr[3];                                                           // :354-355, :381-382
-    vsl[0] = sm;
-    vsr[0] = sm;
-    {
-        const double bxl_dnl = bl[0] / dn_l, bxr_dnr = br[0] / dn_r;
-        vsl[1] = ul[2] + (bxl_dnl * (bl[1] - bsl[1]));
-        vsl[2] = ul[3] + (bxl_dnl * (bl[2] - bsl[2]));
-        vsr[1] = ur[2] + (bxr_dnr * (br[1] - bsr[1]));
-        vsr[2] = ur[3] + (bxr_dnr * (br[2] - bsr[2]));
-    }
-    const double vb_starl = (vsl[0] * bsl[0] + vsl[1] * bsl[1]) + vsl[2] * bsl[2];  // :388-389
-    const double vb_starr = (vsr[0] * bsr[0] + vsr[1] * bsr[1]) + vsr[2] * bsr[2];
-
-    double usl[5], usr[5];                                                           // :393-404
-    usl[0] = dn_l / slsm;
-    usr[0] = dn_r / srsm;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        usl[1 + c] = usl[0] * vsl[c];
-        usr[1 + c] = usr[0] * vsr[c];
-    }
-    if (has_energy) {
-        const double vb_l = (ul[1] * bl[0] + ul[2] * bl[1]) + ul[3] * bl[2];
-        const double vb_r = (ur[1] * br[0] + ur[2] * br[1]) + ur[3] * br[2];
-        usl[4] = ((((slvxl * enl) - (prl * ul[1])) + (prt_star * sm)) + (bl[0] * (vb_l - vb_starl))) / slsm;
-        usr[4] = ((((srvxr * enr) - (prr * ur[1])) + (prt_star * sm)) + (br[0] * (vb_r - vb_starr))) / srsm;
-    }
-
-    // flux through the outer (star) state of one side: fl + s*(u_star - u) (Eq. 64)
-    auto star_flux = [&](bool left, double* out, double* bout) {
-        const double* u = left ? ul : ur;
-        const double* b = left ? bl : br;
-        const double* us = left ? usl : usr;
-        const double* bs = left ? bsl : bsr;
-        const double s = left ? sl : sr;
-        const double en = left ? enl : enr;
-        double fs[5];
-        side_flux(has_energy, u, b, left ? prl : prr, en, fs);
-#pragma unroll
-        for (int c = 0; c < 5; ++c)
-            if (c < nc) out[c] = fs[c] + s * (us[c] - side_cons(u, en, c));
-        bout[0] = side_bflux(u, b, 1) + s * (bs[1] - b[1]);
-        bout[1] = side_bflux(u, b, 2) + s * (bs[2] - b[2]);
-    };
-
-    if (fabs(bl[0]) > 0.0) {                                                         // :410
-        const double dn_lsqt = sqrt(usl[0]);                                        // :414-418
-        const double dn_rsqt = sqrt(usr[0]);
-        const double alfven_l = sm - fabs(bl[0]) / dn_lsqt;
-        const double alfven_r = sm + fabs(br[0]) / dn_rsqt;
-        if (alfven_l > 0.0 || alfven_r < 0.0) {                                      // :422-448
-            star_flux(alfven_l > 0.0, f, bf);
-            return;
-        }
-        const double b_sig = (bl[0] >= 0.0) ? 1.0 : -1.0;                            // :452-456
-        const double add_dnsq = dn_lsqt + dn_rsqt;                                   // :460-461
-        const double mul_dnsq = dn_lsqt * dn_rsqt;
-        double v2[3], b2[3];                                                         // :465-470
-        v2[0] = sm;
-        v2[1] = ((dn_lsqt * vsl[1] + dn_rsqt * vsr[1]) + b_sig * (bsr[1] - bsl[1])) / add_dnsq;
-        v2[2] = ((dn_lsqt * vsl[2] + dn_rsqt * vsr[2]) + b_sig * (bsr[2] - bsl[2])) / add_dnsq;
-        b2[0] = 0.5 * (bl[0] + br[0]);
-        const double bsm = b_sig * mul_dnsq;
-        b2[1] = ((dn_lsqt * bsr[1] + dn_rsqt * bsl[1]) + bsm * (vsr[1] - vsl[1])) / add_dnsq;
-        b2[2] = ((dn_lsqt * bsr[2] + dn_rsqt * bsl[2]) + bsm * (vsr[2] - vsl[2])) / add_dnsq;
-        const double vb_2star = (v2[0] * b2[0] + v2[1] * b2[1]) + v2[2] * b2[2];   // :474
-
-        // flux through the Alfven (2-star) state of one side (Eq. 65, :478-522)
-        auto alfven_flux = [&](bool left, double* out, double* bout) {
-            const double* u = left ? ul : ur;
-            const double* b = left ? bl : br;
-            const double* us = left ? usl : usr;
-            const double* bs = left ? bsl : bsr;
-            const double s = left ? sl : sr;
-            const double en = left ? enl : enr;
-            const double a = left ? alfven_l : alfven_r;
-            double u2[5], fs[5];
-            u2[0] = us[0];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) u2[1 + c] = us[0] * v2[c];
-            if (has_energy)
-                u2[4] = left ? us[4] - (b_sig * dn_lsqt) * (vb_starl - vb_2star)
-                             : us[4] + (b_sig * dn_rsqt) * (vb_starr - vb_2star);
-            side_flux(has_energy, u, b, left ? prl : prr, en, fs);
-#pragma unroll
-            for (int c = 0; c < 5; ++c)
-                if (c < nc) out[c] = ((fs[c] + a * u2[c]) - (a - s) * us[c]) - s * side_cons(u, en, c);
-#pragma unroll
-            for (int c = 1; c < 3; ++c)
-                bout[c - 1] = ((side_bflux(u, b, c) + a * b2[c]) - (a - s) * bs[c]) - s * b[c];
-        };
-        if (sm > 0.0 || sm < 0.0) {                                                  // :496-522
-            alfven_flux(sm > 0.0, f, bf);
-        } else {                                                                     // :524-544
-            double fl2[5], fr2[5], bl2[2], br2[2];
-            alfven_flux(true, fl2, bl2);
-            alfven_flux(false, fr2, br2);
-#pragma unroll
-            for (int c = 0; c < 5; ++c)
-                if (c < nc) f[c] = 0.5 * (fl2[c] + fr2[c]);
-            bf[0] = 0.5 * (bl2[0] + br2[0]);
-            bf[1] = 0.5 * (bl2[1] + br2[1]);
-        }
-    } else {                                                                         // :548-599, B_x = 0
-        if (sm > 0.0 || sm < 0.0) {
-            star_flux(sm > 0.0, f, bf);
-        } else {
-            // half * (fl + sl*(usl-ucl) + fr + sr*(usr-ucr)), summed left to right
-            double fsl[5], fsr[5];
-            side_flux(has_energy, ul, bl, prl, enl, fsl);
-            side_flux(has_energy, ur, br, prr, enr, fsr);
-#pragma unroll
-            for (int c = 0; c < 5; ++c)
-                if (c < nc)
-                    f[c] = 0.5 * (((fsl[c] + sl * (usl[c] - side_cons(ul, enl, c))) + fsr[c]) +
-                                  sr * (usr[c] - side_cons(ur, enr, c)));
-#pragma unroll
-            for (int c = 1; c < 3; ++c)
-                bf[c - 1] = 0.5 * (((side_bflux(ul, bl, c) + sl * (bsl[c] - bl[c])) + side_bflux(ur, br, c)) +
-                                   sr * (bsr[c] - br[c]));
-        }
-    }
+    Ieee ar;
+    const double l[5] = {ul[0], ul[1], ul[2], ul[3], has_energy ? ul[4] : 0.0};
+    const double r[5] = {ur[0], ur[1], ur[2], ur[3], has_energy ? ur[4] : 0.0};
+    const double x[3] = {bl[0], bl[1], bl[2]}, y[3] = {br[0], br[1], br[2]};
+    double o[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, ob[2] = {0.0, 0.0};
+    hlld_face(ar, has_energy, gamma, 0.0, 0.0, l, r, x, y, o, ob);
+    for (int c = 0; c < (has_energy ? 5 : 4); ++c) f[c] = o[c];
+    bf[0] = ob[0];
+    bf[1] = ob[1];
 }
 
 PK_PHYS void hllc_iface(bool has_energy, double gamma, const double* ul, const double* ur, double* f)
 {
-    double fl[5], fr[5], usl[5], usr[5];
-    double prl, prr, c_fastm;
-    double enl = 1.7976931348623157e308, enr = 1.7976931348623157e308;
-    const int nc = has_energy ? 5 : 4;
-    if (gamma < 0.0) {                                                               // hlld.F90:673-677
-        prl = 0.0;
-        prr = 0.0;
-        c_fastm = 0.0;
-    } else {                                                                         // :689-703
-        prl = ul[4];
-        prr = ur[4];
-        enl = (ul[4] / (gamma - 1.0)) + ((0.5 * ul[0]) * ((ul[1] * ul[1] + ul[2] * ul[2]) + ul[3] * ul[3]));
-        enr = (ur[4] / (gamma - 1.0)) + ((0.5 * ur[0]) * ((ur[1] * ur[1] + ur[2] * ur[2]) + ur[3] * ur[3]));
-        const double gampr_l = gamma * ul[4];
-        const double gampr_r = gamma * ur[4];
-        c_fastm = sqrt(f_max(gampr_l / ul[0], gampr_r / ur[0]));
-    }
-    const double sl = f_min(ul[1], ur[1]) - c_fastm;                                // :719-720
-    const double sr = f_max(ul[1], ur[1]) + c_fastm;
-    fl[0] = ul[0] * ul[1];                                                           // :724-734
-    fl[1] = (ul[0] * (ul[1] * ul[1])) + prl;
-    fl[2] = (ul[0] * ul[2]) * ul[1];
-    fl[3] = (ul[0] * ul[3]) * ul[1];
-    if (has_energy) fl[4] = (enl + prl) * ul[1];
-    fr[0] = ur[0] * ur[1];
-    fr[1] = (ur[0] * (ur[1] * ur[1])) + prr;
-    fr[2] = (ur[0] * ur[2]) * ur[1];
-    fr[3] = (ur[0] * ur[3]) * ur[1];
-    if (has_energy) fr[4] = (enr + prr) * ur[1];
-    if (sl >= 0.0) {                                                                 // :738-743
-#pragma unroll
-        for (int c = 0; c < 5; ++c)
-            if (c < nc) f[c] = fl[c];
-        return;
-    }
-    if (sr <= 0.0) {
-#pragma unroll
-        for (int c = 0; c < 5; ++c)
-            if (c < nc) f[c] = fr[c];
-        return;
-    }
-    double sm;                                                                       // :747-754
-    {
-        const double auxr = (sr - ur[1]) * ur[0];
-        const double auxl = (sl - ul[1]) * ul[0];
-        if (fabs(auxr - auxl) < f_spacing(auxr + auxl)) sm = (sl + sr) / 2.0;
-        else sm = ((auxr * ur[1] - prr) - (auxl * ul[1] - prl)) / (auxr - auxl);
-    }
-    const double slvxl = sl - ul[1], srvxr = sr - ur[1];                            // :758-764
-    const double dn_l = ul[0] * slvxl, dn_r = ur[0] * srvxr;
-    const double prt_star = 0.5 * ((prl + dn_l * (sm - ul[1])) + (prr + dn_r * (sm - ur[1])));
-    if (sm >= 0.0) {                                                                 // :771-784
-        const double slsm = sl - sm;
-        usl[0] = dn_l / slsm;
-        usl[1] = usl[0] * sm;
-        usl[2] = usl[0] * ul[2];
-        usl[3] = usl[0] * ul[3];
-        if (has_energy) usl[4] = (((slvxl * enl) - (prl * ul[1])) + (prt_star * sm)) / slsm;
-    }
-    if (sm <= 0.0) {                                                                 // :786-796
-        const double srsm = sr - sm;
-        usr[0] = dn_r / srsm;
-        usr[1] = usr[0] * sm;
-        usr[2] = usr[0] * ur[2];
-        usr[3] = usr[0] * ur[3];
-        if (has_energy) usr[4] = (((srvxr * enr) - (prr * ur[1])) + (prt_star * sm)) / srsm;
-    }
-    double ucl[5], ucr[5];
-    ucl[0] = ul[0];
-    ucr[0] = ur[0];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        ucl[1 + c] = ul[0] * ul[1 + c];
-        ucr[1 + c] = ur[0] * ur[1 + c];
-    }
-    ucl[4] = enl;
-    ucr[4] = enr;
-    if (sm > 0.0) {                                                                  // :798-806
-#pragma unroll
-        for (int c = 0; c < 5; ++c)
-            if (c < nc) f[c] = fl[c] + sl * (usl[c] - ucl[c]);
-    } else if (sm < 0.0) {                                                           // :808-815
-#pragma unroll
-        for (int c = 0; c < 5; ++c)
-            if (c < nc) f[c] = fr[c] + sr * (usr[c] - ucr[c]);
-    } else {                                                                         // :817-829
-#pragma unroll
-        for (int c = 0; c < 5; ++c)
-            if (c < nc) f[c] = 0.5 * (((fl[c] + sl * (usl[c] - ucl[c])) + fr[c]) + sr * (usr[c] - ucr[c]));
-    }
+    Ieee ar;
+    const double l[5] = {ul[0], ul[1], ul[2], ul[3], has_energy ? ul[4] : 0.0};
+    const double r[5] = {ur[0], ur[1], ur[2], ur[3], has_energy ? ur[4] : 0.0};
+    double o[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    hllc_face(ar, has_energy, gamma, 0.0, l, r, o);
+    for (int c = 0; c < (has_energy ? 5 : 4); ++c) f[c] = o[c];
 }
 
 // riemann_wrap / riemann_wrap_u (hlld.F90:62-155) for one interface of the

@@ -103,6 +103,30 @@ struct Roles {
 template <class PH, int S>
 PK_PHYS constexpr size_t tile_doubles() { return (size_t)3 * PH::NV * S; }
 
+template <class PH>
+__device__ __noinline__ void utoq_ieee_mem(const double* u, double* q, const PhysParams& pp)
+{
+    double x[PH::NV], y[PH::NV];
+#pragma unroll
+    for (int v = 0; v < PH::NV; ++v) x[v] = u[v];
+    utoq<PH>(x, y, pp);
+#pragma unroll
+    for (int v = 0; v < PH::NV; ++v) q[v] = y[v];
+}
+
+// utoq in IEEE operations, out of line, for a cell that the branch-free
+// quotients' range does not hold
+template <class PH>
+PK_DEV void utoq_ieee(const double (&u)[PH::NV], double (&q)[PH::NV], const PhysParams& pp)
+{
+    double x[PH::NV], y[PH::NV];
+#pragma unroll
+    for (int v = 0; v < PH::NV; ++v) x[v] = u[v];
+    utoq_ieee_mem<PH>(x, y, pp);
+#pragma unroll
+    for (int v = 0; v < PH::NV; ++v) q[v] = y[v];
+}
+
 // The face states of one cell from its own primitives q and its neighbours'
 // (slots mp, mn) for component planes [V0, V1): q becomes the left state of the
 // cell's right face, the right state of its left face goes to R.  The limiter
@@ -171,7 +195,7 @@ constexpr int KEEP_NV = 9;
 template <class PH, int S, bool REC = false, bool W3 = false, bool FC = false, bool FAST = false, bool U0S = false,
           bool FLUX = false>
 PK_DEV void rk_stage(double* __restrict__ sm, int me, int mp, int mn, const Roles& r, double (&w)[PH::NV],
-                     const double* u0src, const double* wsrc, long long off, const Geom& g, double dtodx, double ch,
+                     const double* u0src, const double* wsrc, long long off, const Geom& g, double dtodx, double ch, double rch,
                      const PhysParams& pp, unsigned& status, FloorRec* rec = nullptr,
                      const double* fc_in = nullptr, double* fc_out = nullptr, const double* u0sm = nullptr,
                      int u0st = 0)
@@ -183,8 +207,13 @@ PK_DEV void rk_stage(double* __restrict__ sm, int me, int mp, int mn, const Role
     double* const F = sm + 2 * NV * S;
     double q[NV];
     if (r.q) {
-        if constexpr (FAST) utoq_fast<PH>(w, q, pp);
-        else utoq<PH>(w, q, pp);
+        if constexpr (FAST) {
+            utoq_fast<PH>(w, q, pp);
+        } else {
+            Exact ar;
+            utoq<PH>(ar, w, q, pp);
+            if (!ar.ok()) utoq_ieee<PH>(w, q, pp);
+        }
 #pragma unroll
         for (int v = 0; v < NV; ++v) Q[v * S + me] = q[v];
     }
@@ -215,7 +244,7 @@ PK_DEV void rk_stage(double* __restrict__ sm, int me, int mp, int mn, const Role
     }
     __syncthreads();
     if (r.flux) {
-        riemann_cell<PH, S, KEEP, FAST>(q, R + mn, F + me, ch, pp);
+        riemann_cell<PH, S, KEEP, FAST>(q, R + mn, F + me, ch, rch, pp);
         if constexpr (FC) {
             if (fc_in) {
 #pragma unroll
@@ -277,6 +306,7 @@ struct StepParams {
     double dt;        // time step
     double ch;        // GLM psi speed (update_chspeed)
     double psi_fac;   // glmdamping factor, applied by the last sweep of each triple
+    double rch;       // 1 / ch, correctly rounded
 };
 
 // floor records of both stages of one cell, as the recording sweep stores
@@ -341,7 +371,7 @@ PK_DEV void fused_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
         r.upd = active && (circ || (t >= a + 2 && t < T - a - 2));
         FloorRec rec{0, 0};
         rk_stage<PH, S, REC, W3, false, FAST>(smem, me, mp, mn, r, w, uin, uin, off, g, stage == 0 ? dtodx1 : dtodx2, ch,
-                                           pp, status, &rec);
+                                           stp.rch, pp, status, &rec);
         if (stage == 0) {
             rec1 = rec;
             if (REC && own) store_cell<PH>(ustar, off, g, w);
@@ -497,7 +527,7 @@ PK_DEV void fc_slots(const FcArgs& fc, const Geom& g, int i1, int i2, int s, con
 
 template <class PH, int S, bool W3, bool FC>
 PK_DEV void stage_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, const double* uin, double* uout,
-                       double* uh, const PhysParams& pp, int first, double dtodx, double ch, const FcArgs& fc,
+                       double* uh, const PhysParams& pp, int first, double dtodx, double ch, double rch, const FcArgs& fc,
                        double* smem, unsigned& status, bool trim = false, bool flat = false)
 {
     constexpr int NV = PH::NV;
@@ -543,8 +573,8 @@ PK_DEV void stage_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
     double* fc_out = nullptr;
     if constexpr (FC)
         if (valid) fc_slots<PH>(fc, g, i1, i2, s, fc_in, fc_out);
-    rk_stage<PH, S, false, W3, FC>(smem, me, me - st, me + st, r, w, first ? uin : uh, uin, off, g, dtodx, ch, pp, status,
-                                nullptr, fc_in, fc_out);
+    rk_stage<PH, S, false, W3, FC>(smem, me, me - st, me + st, r, w, first ? uin : uh, uin, off, g, dtodx, ch, rch, pp,
+                                   status, nullptr, fc_in, fc_out);
     if (own && (!trim || inner)) store_cell<PH>(uout, off, g, w);
 }
 
@@ -560,7 +590,7 @@ __global__ void __launch_bounds__(MAXT) k_stage(Geom g, Tile tl, const double* u
     unsigned status = 0;
     const double dtodx = (rk * spar->dt) / dl;                 // rk_coef(istep) * dt / cg%dl(ddim)
     stage_tile<PH, MAXT, W3, FC>(g, tl, blockIdx.x * tl.P, blockIdx.y * tl.L, blockIdx.z, uin, uout, uh, pp, first, dtodx,
-                           spar->ch, fc, smem, status);
+                           spar->ch, spar->rch, fc, smem, status);
     flush_status(status, gstatus);
 }
 
@@ -608,8 +638,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_stage_batched(const BlockDesc* _
     const double dtodx = (rk * spar->dt) / b.dl[dir];
     const FcArgs fc = fcs ? fcs[w.block] : FcArgs{};
     double* u = const_cast<double*>(b.in);
-    stage_tile<PH, MAXT, W3, FC>(g, tl, w.i1_0, b.g[dir] - 2, w.i2, u, u, b.uh, pp, first, dtodx, spar->ch, fc, smem, status,
-                           true, true);
+    stage_tile<PH, MAXT, W3, FC>(g, tl, w.i1_0, b.g[dir] - 2, w.i2, u, u, b.uh, pp, first, dtodx, spar->ch, spar->rch, fc, smem,
+                           status, true, true);
     flush_status(status, gstatus);
 }
 
@@ -723,8 +753,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_stage_refined(const BlockDesc* _
             const double dtodx = (rk * spar->dt) / b.dl[dir];
             const FcArgs fc = fcs ? fcs[it.block] : FcArgs{};
             double* u = const_cast<double*>(b.in);
-            stage_tile<PH, MAXT, W3, true>(g, tl, it.i1_0, b.g[dir] - 2, 0, u, u, b.uh, pp, first, dtodx, spar->ch, fc,
-                                     smem, status, true, true);
+            stage_tile<PH, MAXT, W3, true>(g, tl, it.i1_0, b.g[dir] - 2, 0, u, u, b.uh, pp, first, dtodx, spar->ch, spar->rch,
+                                     fc, smem, status, true, true);
         } else {
             const long long n = (long long)(it.end - it.beg) * NV;
             for (long long t = threadIdx.x; t < n; t += blockDim.x) {
@@ -796,7 +826,7 @@ __global__ void __launch_bounds__(MAXT, 2) k_unsplit_flux(Geom g, Tile tl, const
     if constexpr (FC)
         if (valid) fc_slots<PH>(fc, g, i1, i2, s, fc_in, fc_out);
     rk_stage<PH, MAXT, false, W3, FC, false, false, true>(smem, me, me - st, me + st, r, w, uin, uin, off, g, 0.0,
-                                                          spar->ch, pp, status, nullptr, fc_in, fc_out);
+                                                          spar->ch, spar->rch, pp, status, nullptr, fc_in, fc_out);
     if (own && r.flux) store_cell<PH>(F, off + g.sd, g, w);
 }
 

@@ -1,0 +1,116 @@
+// pk_quotient.cuh -- correctly rounded quotients without branches.
+//
+// The bit-exact kernels take about 28 quotients per cell and RK stage (MHD).  The
+// compiler's division is a sequence with a conditional slow path: 19 issue
+// slots, 126 cycles of latency, and because each one ends in a branch,
+// independent divisions of a thread do not overlap (measured on B200: 34
+// cycles per warp and division at four warps per scheduler, whether a thread
+// has one or four independent ones in flight; a fused multiply-add takes 2).
+// Exact computes the same bits from a reciprocal per denominator and three
+// operations per quotient, straight-line, and records whether every operand
+// was in the range where that is proven; a thread that was not (a few values
+// beyond 1e77 or nonzero ones below 1e-77) redoes its work with the IEEE
+// operations (the callers' `if (!ar.ok())`).
+//
+// Why the bits are the same (P. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990) 111-119;
+// ulp: unit in the last place of the result, d scaled into [1, 2)):
+//  * y: the hardware's reciprocal approximation (about 20 bits) and three
+//    Newton steps y + y (1 - d y).  After two of them y is less than an ulp off,
+//    so the third's residual 1 - d y is exact and its result is the rounded 1/d:
+//    with the one known exception of d = 2 - 2^-52 reached from below, which
+//    rounding the second step upwards excludes.  So |y - 1/d| <= 2^-54.
+//  * q = n y rounded, r = n - d q (exact by the fused operation, no underflow in
+//    the checked range), result q + r y rounded once.  Before that rounding it
+//    is off n/d by |r| |y - 1/d|.  A wrong rounding needs n/d closer than that to
+//    the midpoint of two neighbours, but n/d stays at least 2^-53 / d ulp away
+//    from every midpoint (n 2^k - d m is a nonzero integer in last places).
+//    Where q is one of the two neighbours, |r| = d / 2 ulp there, and the error
+//    stays below (d^2 / 4) 2^-53 / d ulp, less than the distance as d < 2.  Where
+//    q is a neighbour's neighbour (n < d, n y off n/d by almost an ulp, 1 - 2^-52
+//    at most since n <= 2 - 2^-51), n/d lies 2^-52 ulp beyond the midpoint and the
+//    error is at most 1.5 2^-53 ulp.
+//  * A zero numerator gives a zero; its sign is q's, which is put back.
+// tests/test_gpu_quotient.py compares with CUDA's division over random and
+// adversarial operands.  Measured with utoq and the Riemann solvers on it (one
+// side's energy and flux, too): a step of the 256^3 MHD block 18.0 -> 16.6 ms, of
+// a 64^3 Sedov blast 0.39 -> 0.26 ms, of a 149 x 93 x 70 open gas box 2.25 -> 1.31 ms,
+// of the three-fluid refined blast 28.1 -> 23.3 ms.  (Picking the side before its
+// star state, with fewer quotients and roots still, was slower: 18.4, 31.4 ms; its
+// one chain of dependent operations leaves nothing to overlap.)
+#pragma once
+#include "pk_device.cuh"
+
+namespace pk {
+
+// the hardware's FP64 reciprocal approximation
+PK_DEV double rcp_seed(double x)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    return r;
+}
+
+struct Exact {
+    static constexpr bool FAST = false;
+    unsigned bad = 0;                       // a set top bit: an operand outside [2^-256, 2^256)
+    PK_DEV bool ok() const { return (bad >> 30) == 0; }
+    PK_DEV void need(double x) { bad |= 2u * (unsigned)__double2hiint(x) - ((1023u - 256u) << 21); }
+    PK_DEV void needz(double x)             // the same, or zero
+    {
+        if (x != 0.0) need(x);
+    }
+    PK_DEV double inv(double d)
+    {
+        need(d);
+        const double m = fabs(d);
+        double y = rcp_seed(m);
+        y = fma(y, fma(-m, y, 1.0), y);
+        y = __fma_ru(y, fma(-m, y, 1.0), y);
+        return copysign(fma(y, fma(-m, y, 1.0), y), d);
+    }
+    PK_DEV static double quotient(double n, double d, double y, double& q)
+    {
+        q = n * y;
+        return fma(fma(-d, q, n), y, q);
+    }
+    PK_DEV double quo(double n, double d, double y)
+    {
+        double q;
+        need(n);
+        return quotient(n, d, y, q);
+    }
+    PK_DEV double quoz(double n, double d, double y)
+    {
+        double q;
+        needz(n);
+        const double x = quotient(n, d, y, q);
+        return __hiloint2double((__double2hiint(x) & 0x7fffffff) | (__double2hiint(q) & 0x80000000), __double2loint(x));
+    }
+    PK_DEV double quoc(double n, double d, double y)
+    {
+        need(d);
+        return quoz(n, d, y);
+    }
+    PK_DEV double root(double x, double&) { return sqrt(x); }
+    PK_DEV double over_root(double n, double root, double) { return quo(n, root, inv(root)); }
+};
+
+// the IEEE versions for a thread whose operands left the range: out of line, so
+// that their registers and code stay out of the kernels' way
+// x: ul(5), ur(5), bl(3), br(3); f: fluid fluxes (5), transverse B fluxes (2)
+static __device__ __noinline__ void hlld_ieee(bool has_energy, double gamma, const double* x, double* f)
+{
+    f[4] = 0.0;
+    hlld_iface(has_energy, gamma, x, x + 5, x + 10, x + 13, f, f + 5);
+}
+
+static __device__ __noinline__ void hllc_ieee(bool has_energy, double gamma, const double* x, double* f)
+{
+    f[4] = 0.0;
+    hllc_iface(has_energy, gamma, x, x + 5, f);
+}
+
+static __device__ __noinline__ double divide_ieee(double n, double d) { return n / d; }
+
+}  // namespace pk

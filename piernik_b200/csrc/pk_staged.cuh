@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(S, 512 / S) k_sweep_staged(const __grid_consta
         for (int s = 0; s < 2; ++s) {
             FloorRec rec{0, 0};
             rk_stage<PH, S, REC, false, false, FAST, true>(sm, t, mp, mn, r, w, nullptr, nullptr, 0, g,
-                                                        s == 0 ? dtodx1 : dtodx2, ch, pp, status, &rec, nullptr,
+                                                        s == 0 ? dtodx1 : dtodx2, ch, stp.rch, pp, status, &rec, nullptr,
                                                         nullptr, mine, 2 * n);
             if constexpr (REC) {
                 if (s == 0) {

@@ -1,0 +1,88 @@
+"""The bit-exact kernels' branch-free quotients (pk_quotient.cuh) against
+CUDA's correctly rounded division, bit for bit, wherever they say that the
+operands are in their range, and that they say so for every operand in
+[2^-256, 2^256) and for zero numerators of quoz and quoc.
+
+Operands: random ones; divisors with significands at either end; quotients
+as close to the midpoint of two doubles as they get (n 2^54 - d m = +-1 for an
+odd 54-bit m: m the inverse of d modulo 2^54); and values outside the range,
+which must be refused or divided correctly."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SRC = os.path.join(HERE, "native", "quotient_harness.cu")
+CSRC = os.path.join(HERE, "..", "piernik_b200", "csrc")
+DEPS = [SRC, os.path.join(CSRC, "pk_quotient.cuh"), os.path.join(CSRC, "pk_device.cuh")]
+LIB = os.path.join(HERE, "native", "libquotient_harness.so")
+
+pytestmark = pytest.mark.gpu
+
+
+def _eval(n, d):
+    if not os.path.exists(LIB) or os.path.getmtime(LIB) < max(os.path.getmtime(p) for p in DEPS):
+        subprocess.check_call(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "--fmad=false",
+                               "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-o", LIB, SRC])
+    n, d = np.ascontiguousarray(n, float), np.ascontiguousarray(d, float)
+    out = np.empty((n.size, 7))
+    p = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))  # noqa: E731
+    assert C.CDLL(LIB).quotient_eval(p(n), p(d), n.size, p(out)) == 0
+    return out
+
+
+def _check(n, d, all_ok):
+    o = _eval(n, d)
+    want = o[:, 6].copy().view(np.uint64)
+    for k, name in enumerate(("quo", "quoz", "quoc")):
+        ok = o[:, 3 + k] != 0
+        if all_ok:
+            assert ok[(n != 0) | (k > 0)].all(), name
+        bad = ok & (o[:, k].copy().view(np.uint64) != want) & ((n != 0) | (k > 0))
+        assert not bad.any(), (name, n[bad][:3], d[bad][:3], o[bad][:3])
+
+
+def _scaled(rng, x):
+    return np.ldexp(x * rng.choice([-1.0, 1.0], x.size), rng.integers(-200, 200, x.size))
+
+
+def test_random_and_edge_significands(gpu_lib):
+    rng = np.random.default_rng(5)
+    m = 1 << 20
+    _check(_scaled(rng, 1 + rng.random(m)), _scaled(rng, 1 + rng.random(m)), True)
+    ends = np.concatenate([1 + np.arange(64) * 2.0**-52, 2 - np.arange(1, 65) * 2.0**-52])
+    _check(np.repeat(ends, ends.size), np.tile(ends, ends.size), True)
+    _check(1 + rng.random(ends.size * 4096), np.tile(ends, 4096), True)
+    zeros = np.tile([0.0, -0.0], 4096)
+    _check(zeros, _scaled(rng, 1 + rng.random(zeros.size)), True)
+
+
+def test_quotients_next_to_a_midpoint(gpu_lib):
+    rng = np.random.default_rng(6)
+    n, d = [], []
+    for b in [int(x) | 1 for x in rng.integers(1 << 52, 1 << 53, 40000)] + [(1 << 53) - 1 - 2 * k for k in range(2000)]:
+        inv = pow(b, -1, 1 << 54)
+        for m, r in ((inv, 1), ((1 << 54) - inv, -1)):       # b m = r modulo 2^54
+            a = (b * m - r) >> 54
+            if a > 0 and m >> 53:
+                n.append(float(a))
+                d.append(float(b))
+    assert len(n) > 10000
+    n, d = np.array(n), np.array(d)
+    _check(n, d, True)
+    _check(np.ldexp(n, -60), -d, True)
+
+
+def test_operands_outside_the_range(gpu_lib):
+    edge = [0.0, 5e-324, 1e-310, 2.3e-308, 1e-200, 2.0**-257, 2.0**-256, 1.0, 2.0**255, 2.0**256, 1e200, 1.7e308, np.inf, np.nan]
+    edge = np.array(edge + [-x for x in edge])
+    n, d = np.repeat(edge, edge.size), np.tile(edge, edge.size)
+    o = _eval(n, d)
+    for k in range(3):
+        ok = o[:, 3 + k] != 0
+        assert not ok[~np.isfinite(n) | ~np.isfinite(d) | (d == 0)].any()
+        same = o[:, k].copy().view(np.uint64) == o[:, 6].copy().view(np.uint64)
+        assert same[ok].all()
