@@ -581,9 +581,15 @@ PK_PHYS void riemann(const double (&ql)[PH::NV], const double (&qr)[PH::NV], dou
 }
 
 // internal_sources (+0 added to every fluid component) and care_for_positives
-// on one updated cell; B used for emag is the updated one (b1).
-template <class PH>
-PK_PHYS void sources_and_floors(double (&u)[PH::NV], const PhysParams& pp, unsigned& status)
+// on one updated cell; B used for emag is the updated one (b1).  quotient(n, d):
+// n / d, correctly rounded.
+struct IeeeQuotient {
+    PK_PHYS double operator()(double n, double d) const { return n / d; }
+};
+
+template <class PH, class Quotient = IeeeQuotient>
+PK_PHYS void sources_and_floors(double (&u)[PH::NV], const PhysParams& pp, unsigned& status,
+                                const Quotient& quotient = Quotient())
 {
 #pragma unroll
     for (int c = 0; c < PH::NVF; ++c) u[c] = u[c] + 0.0;
@@ -597,7 +603,7 @@ PK_PHYS void sources_and_floors(double (&u)[PH::NV], const PhysParams& pp, unsig
     for (int f = 0; f < PH::NFL; ++f) {                                   // limit_minimal_intener
         if (!PH::has_en(f)) continue;
         const int b = PH::beg(f);
-        const double kin = (0.5 * ((u[b + 1] * u[b + 1] + u[b + 2] * u[b + 2]) + u[b + 3] * u[b + 3])) / u[b];
+        const double kin = quotient(0.5 * ((u[b + 1] * u[b + 1] + u[b + 2] * u[b + 2]) + u[b + 3] * u[b + 3]), u[b]);
         double mag = 0.0, eint;
         if (PH::magn(f)) {
             const double bx = u[PH::IB], by = u[PH::IB + 1], bz = u[PH::IB + 2];
@@ -622,8 +628,9 @@ struct FloorRec {
     unsigned en;   // bit f: the internal-energy floor of fluid f clipped
 };
 
-template <class PH>
-PK_PHYS void floors_rec(double (&u)[PH::NV], const PhysParams& pp, unsigned& status, FloorRec& rec)
+template <class PH, class Quotient = IeeeQuotient>
+PK_PHYS void floors_rec(double (&u)[PH::NV], const PhysParams& pp, unsigned& status, FloorRec& rec,
+                        const Quotient& quotient = Quotient())
 {
     rec.dn = 0;
     rec.en = 0;
@@ -642,7 +649,7 @@ PK_PHYS void floors_rec(double (&u)[PH::NV], const PhysParams& pp, unsigned& sta
     for (int f = 0; f < PH::NFL; ++f) {
         if (!PH::has_en(f)) continue;
         const int b = PH::beg(f);
-        const double kin = (0.5 * ((u[b + 1] * u[b + 1] + u[b + 2] * u[b + 2]) + u[b + 3] * u[b + 3])) / u[b];
+        const double kin = quotient(0.5 * ((u[b + 1] * u[b + 1] + u[b + 2] * u[b + 2]) + u[b + 3] * u[b + 3]), u[b]);
         double mag = 0.0, eint;
         if (PH::magn(f)) {
             const double bx = u[PH::IB], by = u[PH::IB + 1], bz = u[PH::IB + 2];

@@ -148,7 +148,47 @@ PK_DEV void limited_faces(int lim, const double* __restrict__ Q, double* __restr
         }
     };
     switch (lim) {
-    case L_VANLEER: faces([&](double dl, double dr) { return end == 0 ? half_slope<L_VANLEER>(dl, dr) : 0.0; }); break;
+    case L_VANLEER:
+        // 2 dl dr / (dl + dr) where dl dr > 0, in groups of five components: their
+        // quotients overlap, and a warp in a uniform region skips them together.
+        // Against an IEEE division per component: unsplit step of a 128^3 MHD block
+        // 2.14 -> 2.01 ms, refined blast 23.3 -> 22.8; a 64^3 Sedov blast, at rest
+        // almost everywhere, 0.26 either way (without the joint skip 0.28).
+#pragma unroll
+        for (int v0 = V0; v0 < V1; v0 += 5) {
+            constexpr int G = 5;
+            double n[G], d[G], h[G];
+            bool any = false;
+#pragma unroll
+            for (int k = 0; k < G; ++k) {
+                const int v = v0 + k < V1 ? v0 + k : V1 - 1;
+                const double dl = q[v] - Q[v * S + mp], dr = Q[v * S + mn] - q[v], dcen = dl * dr;
+                const bool up = v0 + k < V1 && end == 0 && dcen > 0.0;
+                n[k] = up ? 2.0 * dcen : 0.0;
+                d[k] = up ? dl + dr : 1.0;
+                h[k] = 0.0;
+                any = any || up;
+            }
+            if (any) {
+                Exact ar;
+#pragma unroll
+                for (int k = 0; k < G; ++k)
+                    if (v0 + k < V1) h[k] = 0.5 * ar.mean(n[k], d[k]);
+                if (!ar.ok()) {
+#pragma unroll
+                    for (int k = 0; k < G; ++k)
+                        if (v0 + k < V1) h[k] = 0.5 * divide_ieee(n[k], d[k]);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < G; ++k)
+                if (v0 + k < V1) {
+                    const double qc = q[v0 + k];
+                    q[v0 + k] = qc + h[k];
+                    R[(v0 + k) * S + me] = qc - h[k];
+                }
+        }
+        break;
     case L_MINMOD: faces([](double dl, double dr) { return half_slope<L_MINMOD>(dl, dr); }); break;
     case L_MONCEN: faces([](double dl, double dr) { return half_slope<L_MONCEN>(dl, dr); }); break;
     default: faces([](double dl, double dr) { return half_slope<L_SUPERBEE>(dl, dr); }); break;
@@ -283,8 +323,8 @@ PK_DEV void rk_stage(double* __restrict__ sm, int me, int mp, int mn, const Role
         load_cell<PH>(wsrc, off, g, w);
     }
     if (r.upd || r.keep) {
-        if constexpr (REC) floors_rec<PH>(w, pp, status, *rec);
-        else sources_and_floors<PH>(w, pp, status);
+        if constexpr (REC) floors_rec<PH>(w, pp, status, *rec, ExactQuotient());
+        else sources_and_floors<PH>(w, pp, status, ExactQuotient());
     }
 }
 

@@ -8,9 +8,9 @@
 // has one or four independent ones in flight; a fused multiply-add takes 2).
 // Exact computes the same bits from a reciprocal per denominator and three
 // operations per quotient, straight-line, and records whether every operand
-// was in the range where that is proven; a thread that was not (a few values
-// beyond 1e77 or nonzero ones below 1e-77) redoes its work with the IEEE
-// operations (the callers' `if (!ar.ok())`).
+// was in the range where that is proven; a thread that was not (numerators
+// beyond 1e77 or nonzero ones below 1e-231, denominators beyond 7e75 or below
+// 5e-79) redoes its work with the IEEE operations (the callers' `if (!ar.ok())`).
 //
 // Why the bits are the same (P. Markstein, "Computation of elementary functions
 // on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34 (1990) 111-119;
@@ -53,16 +53,26 @@ PK_DEV double rcp_seed(double x)
 
 struct Exact {
     static constexpr bool FAST = false;
-    unsigned bad = 0;                       // a set top bit: an operand outside [2^-256, 2^256)
-    PK_DEV bool ok() const { return (bad >> 30) == 0; }
-    PK_DEV void need(double x) { bad |= 2u * (unsigned)__double2hiint(x) - ((1023u - 256u) << 21); }
-    PK_DEV void needz(double x)             // the same, or zero
+    // |n| in [2^-768, 2^256) and |d| in [2^-260, 2^252) keep every intermediate and
+    // the quotient normal.  t = 2 x high word holds the exponent in its upper 11 bits:
+    // a numerator outside its range sets the top bit of bad_n, a denominator one
+    // of the two top bits of bad_d.
+    unsigned bad_n = 0, bad_d = 0;
+    PK_DEV static unsigned twice(double x) { return 2u * (unsigned)__double2hiint(x); }
+    PK_DEV bool ok() const { return (((bad_n >> 1) | bad_d) >> 30) == 0; }
+    PK_DEV void need(double n) { bad_n |= twice(n) - ((1023u - 768u) << 21); }
+    PK_DEV void needz(double n)             // the same, or zero
     {
-        if (x != 0.0) need(x);
+        if (n != 0.0) need(n);
     }
+    PK_DEV void needd(double d) { bad_d |= twice(d) - ((1023u - 260u) << 21); }
     PK_DEV double inv(double d)
     {
-        need(d);
+        needd(d);
+        return rounded_inverse(d);
+    }
+    PK_DEV static double rounded_inverse(double d)
+    {
         const double m = fabs(d);
         double y = rcp_seed(m);
         y = fma(y, fma(-m, y, 1.0), y);
@@ -87,9 +97,18 @@ struct Exact {
         const double x = quotient(n, d, y, q);
         return __hiloint2double((__double2hiint(x) & 0x7fffffff) | (__double2hiint(q) & 0x80000000), __double2loint(x));
     }
+    // van Leer's quotient 2 a b / (a + b) for a b > 0: between a and b and twice
+    // that, so n in [2^-900, 2^124) and d < 2^100 suffice (d is at least sqrt(2 n)), and the
+    // fading differences ahead of a front stay in range; n = 0, d = 1 elsewhere
+    PK_DEV double mean(double n, double d)
+    {
+        double q;
+        if (n != 0.0) bad_n |= (twice(n) - ((1023u - 900u) << 21)) | (twice(d) - ((1023u - 924u) << 21));
+        return quotient(n, d, rounded_inverse(d), q);
+    }
     PK_DEV double quoc(double n, double d, double y)
     {
-        need(d);
+        needd(d);
         return quoz(n, d, y);
     }
     PK_DEV double root(double x, double&) { return sqrt(x); }
@@ -112,5 +131,15 @@ static __device__ __noinline__ void hllc_ieee(bool has_energy, double gamma, con
 }
 
 static __device__ __noinline__ double divide_ieee(double n, double d) { return n / d; }
+
+// n / d, correctly rounded: the floors' quotient
+struct ExactQuotient {
+    PK_DEV double operator()(double n, double d) const
+    {
+        Exact ar;
+        const double x = ar.quoz(n, d, ar.inv(d));
+        return ar.ok() ? x : divide_ieee(n, d);
+    }
+};
 
 }  // namespace pk

@@ -1,7 +1,9 @@
 """The bit-exact kernels' branch-free quotients (pk_quotient.cuh) against
 CUDA's correctly rounded division, bit for bit, wherever they say that the
-operands are in their range, and that they say so for every operand in
-[2^-256, 2^256) and for zero numerators of quoz and quoc.
+operands are in their range, and that they say so for numerators in
+[2^-768, 2^256), denominators in [2^-260, 2^252) and zero numerators of quoz
+and quoc.  Van Leer's mean 2 a b / (a + b) (mean) alike, for 2 a b in [2^-900, 2^124)
+and a + b < 2^100.
 
 Operands: random ones; divisors with significands at either end; quotients
 as close to the midpoint of two doubles as they get (n 2^54 - d m = +-1 for an
@@ -28,7 +30,7 @@ def _eval(n, d):
         subprocess.check_call(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "--fmad=false",
                                "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-o", LIB, SRC])
     n, d = np.ascontiguousarray(n, float), np.ascontiguousarray(d, float)
-    out = np.empty((n.size, 7))
+    out = np.empty((n.size, 9))
     p = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))  # noqa: E731
     assert C.CDLL(LIB).quotient_eval(p(n), p(d), n.size, p(out)) == 0
     return out
@@ -58,6 +60,30 @@ def test_random_and_edge_significands(gpu_lib):
     _check(1 + rng.random(ends.size * 4096), np.tile(ends, 4096), True)
     zeros = np.tile([0.0, -0.0], 4096)
     _check(zeros, _scaled(rng, 1 + rng.random(zeros.size)), True)
+
+
+def test_far_ends_of_the_range(gpu_lib):
+    rng = np.random.default_rng(8)
+    m = 1 << 18
+    n = np.ldexp(1 + rng.random(m), rng.choice([-768, -767, -700, 254, 255], m))
+    d = np.ldexp(1 + rng.random(m), rng.choice([-260, -259, 250, 251], m))
+    _check(n, d, True)
+
+
+def test_van_leer_mean(gpu_lib):
+    rng = np.random.default_rng(9)
+    m = 1 << 18
+    a = np.ldexp(1 + rng.random(m), rng.integers(-440, 60, m))
+    b = np.where(rng.random(m) < 0.5, a * (1 + 1e-3 * rng.random(m)), np.ldexp(1 + rng.random(m), rng.integers(-440, 60, m)))
+    s = rng.choice([-1.0, 1.0], m)
+    n, d = 2.0 * (a * b), s * (a + b)
+    o = _eval(n, d)
+    assert (o[:, 8] != 0).all()
+    assert np.array_equal(o[:, 7].copy().view(np.uint64), o[:, 6].copy().view(np.uint64))
+    zero = _eval(np.zeros(4), np.ones(4))
+    assert (zero[:, 8] != 0).all() and (zero[:, 7].copy().view(np.uint64) == 0).all()
+    far = _eval([2.0**-950, 2.0**150, np.inf, np.nan, 2.0**100], [2.0**-470, 2.0**100, np.inf, 1.0, np.nan])
+    assert (far[:, 8] == 0).all()
 
 
 def test_quotients_next_to_a_midpoint(gpu_lib):
