@@ -621,9 +621,11 @@ int refresh_guards(pk_ctx* h, Block& b)
 // A connected domain sweeps with the fused kernels when the blocks tile a
 // domain periodic in every swept direction: the exchange before each sweep
 // then fills every guard cell, and the kernels read their 4-cell halo from
-// the guards -- the same values a periodic single block reads by wrapping.
+// the guards -- the same values a periodic single block reads by wrapping.  With
+// fewer than four guard layers the sweeps go stage by stage.
 bool connected_fused_ok(pk_ctx* h)
 {
+    if (h->cfg.nb < 4) return false;
     long long cells = 0;
     for (auto& b : h->blocks) {
         if (!b.placed) return false;

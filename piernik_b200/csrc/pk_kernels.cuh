@@ -382,9 +382,11 @@ PK_DEV void fused_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
     const int pstride = tl.xfast ? T : 1, st = tl.xfast ? 1 : P;
     const int me = p * pstride + t * st;
     const int i1 = i1_0 + p;
-    const bool active = (tid < PT) && (i1 < g.n1);
     const bool circ = tl.circ;
     const int s = circ ? c0 + t : c0 - 4 + t;                  // position along the pencil (interior coords)
+    // a tile that ends beyond the pencil wraps round, or stops at the four guard
+    // cells that the exchange filled: there is nothing of the block behind them
+    const bool active = (tid < PT) && (i1 < g.n1) && (tl.wrap || s < g.n_d + 4);
     const long long off = (long long)(g.g_d + (tl.wrap ? wrap(s, g.n_d) : s)) * g.sd + (long long)(g.g1 + i1) * g.s1 +
                           (long long)(g.g2 + i2) * g.s2;
     const int mp = circ ? p * pstride + (t == 0 ? T - 1 : t - 1) * st : me - st;
