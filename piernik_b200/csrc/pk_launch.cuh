@@ -145,9 +145,65 @@ int set_smem_attr(pk_ctx* h)
     return PK_OK;
 }
 
+constexpr size_t STAGED_SMEM_SM = 228 * 1024;      // shared memory of one SM (1 KB of it per resident CTA)
 constexpr int DEF_VARIANT[3] = {0, 0, 0};
 constexpr int DEF_P[3] = {2, 4, 4};
 constexpr int DEF_L[3] = {64, 64, 64};
+
+// The tile of a sweep that no one tuned (pk_set_tile).  Measured on B200 per sweep
+// against the one fixed tile for all sizes (320 threads, 2 or 4 pencils x 64
+// cells), bit-exact MHD unless said, us (x / y / z):
+//   the TMA-staged whole pencils wherever they can run and fill the chip with at
+//   least 12 warps per SM (two pencils per CTA, in turn, are too few CTAs below:
+//   32^3 21.8 against 17.7):  64^3 57 / 71 / 72 -> 50 / 52 / 52, 100^3 344 / 357 / 368
+//   -> 194 / 190 / 190, 128^3 561 / 589 / 609 -> 308 / 306 / 307, 128^3 gas 220 / 324 /
+//   337 -> 143 / 148 / 148;
+//   elsewhere whole pencils in 256-thread CTAs, two per SM, where they fit (for
+//   y and z with four or more neighbouring pencils, so that loads coalesce):
+//   75 x 51 x 33 70 / 55 / 49 -> 37 / 41 / 41, 32^3 23 / 18 / 18 -> 18 / 18 / 17,
+//   256 x 256 x 1 x 28 -> 20;
+//   longer ones in equal chunks: along x 128-thread CTAs of one pencil, 512 x 512 x 1
+//   74 -> 60; along y and z 192-thread CTAs of four, 84 -> 68.
+// Stacked instances sweep z in whole segments, which 512-thread CTAs hold best.
+// Blocks below 32^3 cells are bound by the latency of one tile and keep the
+// fixed tile (16^3: 14 us either way), as does a connected domain's one block.
+inline void default_tile(const Block& b, int dir, const Geom& g, int nplanes, bool wrap, bool staged, int* P, int* L,
+                         int* var)
+{
+    const long long cells = (long long)b.n[0] * b.n[1] * b.n[2];
+    if (!wrap || cells < 32768) return;
+    const bool along = g.seg_len && g.seg_along;
+    const int n = along ? g.seg_len : b.n[dir];
+    if (staged && staged_ok(b.n, b.g, b.ext, nplanes, dir, g.seg_len)) {
+        const int threads = (n + 31) / 32 * 32;
+        const int per_sm = std::min((int)(STAGED_SMEM_SM / (staged_smem(nplanes, n) + 1024)), 512 / staged_stride(n));
+        const long long pairs = (long long)((g.n1 + 1) / 2) * g.n2;
+        if (per_sm * threads >= 384 && pairs * threads >= 384LL * sm_count()) {
+            *P = 2;
+            *L = n;
+            *var = VAR_STAGED;
+            return;
+        }
+    }
+    const int whole = VAR_T[2] / n;                   // whole pencils per 256-thread CTA
+    if (dir == 0 ? whole >= 1 : (whole >= 4 || (whole >= 1 && g.n1 <= whole))) {
+        *var = 2;
+        *P = whole;
+        *L = n;
+        return;
+    }
+    if (along) {
+        *var = 6;
+        *P = VAR_T[6] / n;
+        *L = n;
+        return;
+    }
+    const int most = dir == 0 ? 88 : 40;              // owned cells per chunk
+    const int chunks = (n + most - 1) / most;
+    *var = dir == 0 ? 3 : 5;
+    *P = dir == 0 ? 1 : 4;
+    *L = (n + chunks - 1) / chunks;
+}
 
 // Tile, grid and variant of the fused sweep along dir (the handle's tuned or
 // default settings; a whole periodic pencil runs without halo when it fits).
@@ -156,12 +212,16 @@ constexpr int DEF_L[3] = {64, 64, 64};
 inline int fused_geometry(pk_ctx* h, const Block& b, int dir, const Geom& g, Tile* tl, dim3* grid, int* var_out,
                           bool staged = false)
 {
-    int L = h->tileL[dir] > 0 ? h->tileL[dir] : DEF_L[dir];
-    if (L > b.n[dir]) L = b.n[dir];
-    int P = h->tileP[dir] > 0 ? h->tileP[dir] : DEF_P[dir];
-    if (P > g.n1) P = g.n1;
-    int var = h->pp.weno3 ? W3_VARIANT : (h->tileV[dir] >= 0 ? h->tileV[dir] : DEF_VARIANT[dir]);
     tl->wrap = h->connected ? 0 : 1;
+    int P = DEF_P[dir], L = DEF_L[dir], var = DEF_VARIANT[dir];
+    if (h->tileP[dir] <= 0 && h->tileL[dir] <= 0 && h->tileV[dir] < 0)
+        default_tile(b, dir, g, h->nplanes, tl->wrap != 0, staged, &P, &L, &var);
+    if (h->tileL[dir] > 0) L = h->tileL[dir];
+    if (L > b.n[dir]) L = b.n[dir];
+    if (h->tileP[dir] > 0) P = h->tileP[dir];
+    if (P > g.n1) P = g.n1;
+    if (h->tileV[dir] >= 0) var = h->tileV[dir];
+    if (h->pp.weno3) var = W3_VARIANT;
     if (var == VAR_STAGED) {
         if (staged && tl->wrap && staged_ok(b.n, b.g, b.ext, h->nplanes, dir, g.seg_len)) {
             tl->P = 2;
