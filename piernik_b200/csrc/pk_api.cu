@@ -127,6 +127,7 @@ int fill_guards_block(pk_ctx* h, Block& b)
 {
     if (int rc = fill_guards_ptr(h, b, state(h, b))) return rc;
     b.guards_stale = false;
+    b.guards_ruled = true;
     return PK_OK;
 }
 
@@ -909,6 +910,21 @@ int glm_scale(pk_ctx* h, double fac)
     return PK_OK;
 }
 
+// Whether the one-launch sweep with boundary rules serves direction dir of a
+// block that fused_ok refuses: a single gas block, RK2, limited slopes, pencils
+// that fit its CTA, guard cells that hold what the rules say (pk_upload and
+// pk_solve_cg leave others, which the stage path reads as they are).
+bool open_block(pk_ctx* h)
+{
+    return !h->connected && h->blocks.size() == 1 && !h->cfg.magnetic && h->cfg.integration_order == 2 &&
+           !h->pp.weno3 && h->ninst == 1 && h->blocks[0].level == 0;
+}
+
+bool open_ok(pk_ctx* h, int dir)
+{
+    return open_block(h) && h->blocks[0].guards_ruled && h->blocks[0].n[dir] > 1 && h->blocks[0].n[dir] + 4 <= OPEN_T;
+}
+
 // sweep(cdim) of all blocks; the step scalars are already in d_step.
 // apply_fac: the psi damping of glmdamping is folded into this sweep.
 // next_dir: the direction the following sweep of the same step takes (-1:
@@ -935,6 +951,16 @@ int sweep_impl(pk_ctx* h, int dir, double dt, double ch, int apply_fac, double f
         h->cur ^= 1;
         return PK_OK;
     }
+    if (open_ok(h, dir)) {
+        if (int rc = ensure_pingpong(h)) return rc;
+        if (int rc = ops->open(h, h->blocks[0], dir)) return rc;
+        h->cur ^= 1;
+        return PK_OK;
+    }
+    if (!h->connected)                                 // the stages read the guard cells
+        for (auto& b : h->blocks)
+            if (b.guards_stale)
+                if (int rc = fill_guards_block(h, b)) return rc;
     const int nst = h->cfg.integration_order == 1 ? 1 : 2;
     if (int rc = exchange_prepare(h)) return rc;       // a refined domain's couplings
     if (h->blocks.size() > 1)
@@ -1467,6 +1493,7 @@ int pk_upload(pk_handle h, int32_t id, const double* u, const double* bf, const 
         return fail(h, PK_E_ARG, "unknown layout");
     }
     b->guards_stale = false;
+    b->guards_ruled = false;                            // whatever the caller put there
     return PK_OK;
 }
 
@@ -1524,6 +1551,7 @@ int pk_solve_cg(pk_handle h, int32_t id, int32_t ddim, int32_t istep, double dt,
     if (!b->uh) PK_CUDA(h, cudaMalloc(&b->uh, sizeof(double) * h->nplanes * b->plane));
     if (stage_chunked(*b, dir))
         if (int rc = ensure_pingpong(h)) return rc;
+    b->guards_ruled = false;                            // the stage updates or keeps the guard cells of its pencils
     if (int rc = put_step_params(h, dt, chspeed, 1.0)) return rc;   // rk_coef(istep) * dt / cg%dl(ddim) on the device
     return ops_of(h)->stage(h, *b, dir, first, rk);
 }
@@ -1901,7 +1929,10 @@ static int clamp_dt(const pk_config& c, pk_time_state& ts, double dt, double c_a
 // CUDA graph captured once (use_graph) or launched one by one
 static int run_step_sweeps(pk_ctx* h, double dt, double ch, double fac)
 {
-    if (h->use_graph && !h->profiling && !h->halo_cb) {
+    // a first step from guard cells of the caller's own is launched one by one
+    // (the captured step finds those that its own sweeps leave)
+    const bool own = open_block(h) && !fused_ok(h) && !h->blocks[0].guards_ruled;
+    if (h->use_graph && !h->profiling && !h->halo_cb && !own) {
         if (int rc = exchange_prepare(h)) return rc;
         if (h->blocks.size() > 1)
             if (int rc = build_batch(h)) return rc;   // tables are built outside the capture
@@ -1909,12 +1940,20 @@ static int run_step_sweeps(pk_ctx* h, double dt, double ch, double fac)
         for (auto& b : h->blocks)
             if (!b.uh && !fused_ok(h)) PK_CUDA(h, cudaMalloc(&b.uh, sizeof(double) * h->nplanes * b.plane));
         if (int rc = eglm_alloc(h)) return rc;
+        if (h->graph_exec && h->graph_cur != h->cur) invalidate_graph(h);   // it reads the other parity's buffer
         if (!h->graph_exec) {
+            h->graph_cur = h->cur;
             // capture the sweeps of one step once; the step scalars are read from d_step
             const int cur0 = h->cur;
             const long long l0 = h->launches;
             PK_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+            const bool stale0 = h->blocks.empty() ? false : h->blocks[0].guards_stale;
+            if (open_block(h)) h->blocks[0].guards_stale = true;   // the captured step refreshes what its stages read
             const int rc = step_sweeps(h, dt, ch, fac);
+            if (open_block(h)) {
+                h->graph_stale = h->blocks[0].guards_stale;
+                h->blocks[0].guards_stale = stale0;
+            }
             h->graph_kernels = h->launches - l0;
             h->launches = l0;                 // counted when the graph is launched
             cudaGraph_t g = nullptr;
@@ -1932,6 +1971,8 @@ static int run_step_sweeps(pk_ctx* h, double dt, double ch, double fac)
         h->launches += h->graph_kernels;
         if (fused_ok(h))
             for (auto& b : h->blocks) b.guards_stale = true;
+        else if (open_block(h))
+            h->blocks[0].guards_stale = h->graph_stale;
         return PK_OK;
     }
     return step_sweeps(h, dt, ch, fac);
@@ -1953,6 +1994,8 @@ static int unsplit_sweep(pk_ctx* h)
         if (int rc = exchange_prepare(h)) return rc;
     }
     for (auto& b : h->blocks) {
+        if (!h->connected && b.guards_stale)           // split sweeps before, on the same handle
+            if (int rc = fill_guards_block(h, b)) return rc;
         if (!h->connected && !b.uh) PK_CUDA(h, cudaMalloc(&b.uh, sizeof(double) * h->nplanes * b.plane));
         for (int d = 0; d < 3; ++d)
             if (b.n[d] > 1 && !b.flux[d]) PK_CUDA(h, cudaMalloc(&b.flux[d], sizeof(double) * h->nplanes * b.plane));
@@ -2188,7 +2231,12 @@ static int retry_copy(pk_ctx* h, int restore)
             if (int rc = refresh_guards(h, b)) return rc;
         if (restore) PK_CUDA(h, cudaMemcpyAsync(state(h, b), b.retry, bytes, cudaMemcpyDeviceToDevice, h->stream));
         else PK_CUDA(h, cudaMemcpyAsync(b.retry, state(h, b), bytes, cudaMemcpyDeviceToDevice, h->stream));
-        if (restore) b.guards_stale = false;
+        if (restore) {
+            b.guards_stale = false;
+            b.guards_ruled = b.retry_ruled;
+        } else {
+            b.retry_ruled = b.guards_ruled;
+        }
     }
     return PK_OK;
 }

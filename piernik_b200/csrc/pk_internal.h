@@ -30,6 +30,7 @@ constexpr int UNSPLIT_MAXT = 256;     // threads per CTA of the unsplit flux ker
 constexpr int NSTAGE_VARIANT = 4;
 constexpr int SV_T[NSTAGE_VARIANT] = {320, 128, 192, 384};
 constexpr int SV_B[NSTAGE_VARIANT] = {1, 3, 2, 1};
+constexpr int OPEN_T = 256;           // threads per CTA of the sweep with boundary rules (two CTAs per SM)
 constexpr int W3_VARIANT = 2;          // interpol_str = 'weno3' runs this launch-bound variant only
 
 struct Block {
@@ -41,7 +42,9 @@ struct Block {
     double* uh = nullptr;                  // stage path: state at the start of the step (cg%w(uh))
     double* stage = nullptr;               // host-layout conversion buffer
     bool guards_stale = false;             // fused sweeps read periodic images and never store guards
+    bool guards_ruled = false;             // the guard cells, unless stale, are what the block's own rules make of the interior
     double* retry = nullptr;               // copy of the state at the start of a step (cflcontrol = redo)
+    bool retry_ruled = false;              // guards_ruled of that copy
     int seg_len = 0;                       // independent instances stacked along z: cells per instance
     long long off[3] = {0, 0, 0};          // first interior cell on the level's cell grid (connected domains)
     bool placed = false;
@@ -158,6 +161,8 @@ struct pk_ctx {
     cudaGraphExec_t graph_exec = nullptr;
     int use_graph = 0;
     long long graph_kernels = 0;        // kernel nodes of the captured step
+    int graph_cur = 0;                  // the parity whose state the captured step reads
+    bool graph_stale = false;           // the captured step of a block with boundary rules leaves its guards stale
     // same-level domain of connected blocks (pk_set_domain / pk_block_place)
     bool connected = false;
     long long dom[3] = {1, 1, 1};
@@ -244,6 +249,7 @@ struct PhysOps {
     int nv;
     int (*prepare)(pk_ctx* h);      // kernel attributes; called before any launch or graph capture
     int (*fused)(pk_ctx* h, Block& b, int dir, int apply_fac);
+    int (*open)(pk_ctx* h, Block& b, int dir);      // a sweep of pencils with boundary rules (gas only)
     int (*stage)(pk_ctx* h, Block& b, int dir, int first, double rk);           // dt, ch from d_step
     int (*stage_batched)(pk_ctx* h, int dir, int level, int first, double rk);  // all blocks of a level
     int (*stage_refined)(pk_ctx* h, int dir, int first, double rk);             // all levels, one launch

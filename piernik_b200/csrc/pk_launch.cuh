@@ -121,6 +121,9 @@ int set_smem_attr(pk_ctx* h)
     static bool done = false;
     if (!done) {
         if (int rc = set_fused_attr<PH, false>(h)) return rc;
+        if constexpr (!PH::MHD)
+            PK_CUDA(h, cudaFuncSetAttribute(k_sweep_open<PH, OPEN_T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            220 * 1024));
         PK_CUDA(h, cudaFuncSetAttribute(k_stage<PH, STAGE_MAXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         PK_CUDA(h, cudaFuncSetAttribute(k_stage<PH, STAGE_MAXT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         220 * 1024));
@@ -296,6 +299,37 @@ int launch_fused(pk_ctx* h, Block& b, int dir, int apply_fac)
     if (int rc = launch_fused_ptr<PH, FAST>(h, b, dir, apply_fac, b.buf[h->cur], b.buf[1 - h->cur])) return rc;
     b.guards_stale = true;
     return PK_OK;
+}
+
+// The fused sweep of a gas block whose pencils (at most OPEN_T - 4 cells) end in
+// boundary rules
+template <class PH>
+int launch_open(pk_ctx* h, Block& b, int dir)
+{
+    if constexpr (PH::MHD) {
+        return fail(h, PK_E_UNSUPPORTED, "boundary rules are for unmagnetised blocks");
+    } else {
+        Geom g = make_geom(b, dir);
+        Tile tl;
+        tl.T = tl.L = b.n[dir] + 4;
+        tl.P = OPEN_T / tl.T;
+        if (tl.P < 1) return fail(h, PK_E_ARG, "pencil longer than the CTA");
+        if (tl.P > g.n1) tl.P = g.n1;
+        tl.halo = 2;
+        tl.xfast = dir == 0;
+        dim3 grid((g.n1 + tl.P - 1) / tl.P, 1, g.n2);
+        const size_t smem = 3ull * PH::NV * OPEN_T * sizeof(double);
+        std::pair<cudaEvent_t, cudaEvent_t> ev;
+        if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
+        k_sweep_open<PH, OPEN_T, 2><<<grid, tl.P * tl.T, smem, h->stream>>>(
+            g, tl, b.bnd[dir][0], b.bnd[dir][1], b.buf[h->cur], b.buf[1 - h->cur], h->pp, b.dl[dir], h->d_step,
+            h->d_status);
+        PK_CUDA(h, cudaGetLastError());
+        if (int rc = ev_end(h, ev)) return fail(h, rc, "cudaEventRecord failed");
+        h->launches += 1;
+        b.guards_stale = true;
+        return PK_OK;
+    }
 }
 
 template <class PH>
@@ -725,7 +759,8 @@ const FastOps* make_fast_ops()
 template <class PH>
 const PhysOps* make_ops()
 {
-    static PhysOps o{PH::NV, set_smem_attr<PH>, launch_fused<PH>, launch_stage<PH>, launch_stage_batched<PH>,
+    static PhysOps o{PH::NV, set_smem_attr<PH>, launch_fused<PH>, launch_open<PH>, launch_stage<PH>,
+                     launch_stage_batched<PH>,
                      launch_stage_refined<PH>, launch_batched<PH>, launch_fused_ptr<PH>, launch_fused_rec<PH>, launch_adj<PH>,
                      launch_unsplit_flux<PH>, launch_unsplit_apply<PH>};
     return &o;
