@@ -144,7 +144,10 @@ struct pk_ctx {
     bool refined_one_launch = false;            // pk_set_refined_launch
     double* d_eglm = nullptr;                   // E-GLM scratch: divB and grad(psi), 4 planes of the largest block
     long long eglm_plane = 0;
-    int stage_variant = 0;                      // launch-bound variant of k_stage_batched (SV_T / SV_B)
+    // launch-bound variant of k_stage_batched (SV_T / SV_B): 384 x 1, twelve warps at 168
+    // registers, which hold the solver almost without spills; refined three-fluid
+    // blast per pass 20.6 ms (320 x 1: 22.0, 128 x 3: 24.2, 192 x 2: 21.1)
+    int stage_variant = 3;
     pk::FcArgs* d_fcargs[3] = {nullptr, nullptr, nullptr};   // per block flux couplings (refined domains)
     pk_time_state ts;
     std::string err;
