@@ -146,7 +146,9 @@ int fill_guards_ptr(pk_ctx* h, Block& b, double* u)
     }
     a.nfl = h->cfg.nfluids;
     a.nplanes = h->nplanes;
-    k_fill_guards<<<grid1d(b.plane, 256), 256, 0, h->stream>>>(box_of(b), u, a);
+    const long long rows = (long long)b.ext[1] * b.ext[2];
+    const int parts = rows < 8192 ? (b.ext[0] + 31) / 32 : 1;   // enough warps for a block of few rows
+    k_fill_guards<<<grid1d(rows * parts * 32, 256), 256, 0, h->stream>>>(box_of(b), u, a, parts);
     PK_CUDA(h, cudaGetLastError());
     h->launches += 1;
     return PK_OK;

@@ -327,10 +327,13 @@ __device__ __forceinline__ int map_guard(int i, int n, int g, int side_lo, int s
 // a plane at a time (51 us for a 128^3 MHD block), a step of a 149 x 93 x 70 open
 // gas box, which refreshes its guards after every stage, took 1.28 ms, an unsplit
 // step of a 128^3 MHD block 2.01; with this they take 1.23 and 1.94.
-static __global__ void __launch_bounds__(256) k_fill_guards(BoxGeom b, double* __restrict__ u, GuardArgs a)
+// parts: warps per row that lies outside; more than one where the block has few
+// rows (a 313 x 100 plane's 100: 2 us more a refresh with one).
+static __global__ void __launch_bounds__(256) k_fill_guards(BoxGeom b, double* __restrict__ u, GuardArgs a, int parts)
 {
-    const int lane = threadIdx.x & 31, rows = b.ext[1] * b.ext[2], nx = b.ext[0], g2 = 2 * b.g[0];
-    for (int row = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); row < rows; row += (int)((gridDim.x * blockDim.x) >> 5)) {
+    const int lane = threadIdx.x & 31, items = b.ext[1] * b.ext[2] * parts, nx = b.ext[0], g2 = 2 * b.g[0];
+    for (int it = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); it < items; it += (int)((gridDim.x * blockDim.x) >> 5)) {
+        const int row = it / parts, part = it - row * parts;
         const int j = row % b.ext[1], k = row / b.ext[1];
         const bool cross = j >= b.g[1] && j < b.g[1] + b.n[1] && k >= b.g[2] && k < b.g[2] + b.n[2];
         bool fl[3] = {false, false, false};
@@ -348,7 +351,7 @@ static __global__ void __launch_bounds__(256) k_fill_guards(BoxGeom b, double* _
             return m;
         };
         if (cross) {
-            if (g2 == 0) continue;
+            if (g2 == 0 || part) continue;
             const int per = g2 <= 32 ? 32 / g2 : 1;            // planes a pass
             for (int c = lane % (g2 <= 32 ? g2 : 32); c < g2; c += 32) {
                 if (lane >= per * g2 && g2 <= 32) break;
@@ -363,7 +366,7 @@ static __global__ void __launch_bounds__(256) k_fill_guards(BoxGeom b, double* _
             }
             continue;
         }
-        for (int i = lane; i < nx; i += 32) {
+        for (int i = part * 32 + lane; i < nx; i += 32 * parts) {
             bool fx = false;
             const int si = map_guard(i, b.n[0], b.g[0], a.bnd[0][0], a.bnd[0][1], fx);
             const unsigned m = turned(fx, fl[1], fl[2]);
