@@ -97,6 +97,28 @@ struct Roles {
     bool keep;     // not updated but kept (pencil end cell): u1 = u, then floors
 };
 
+// Positions [0, end) of a fused tile's pencil of T cells hold cells of the block:
+// all of them where the pencil wraps round, else those up to the four guard cells
+// that the exchange filled behind a pencil of n cells (there is nothing of the
+// block behind them).  c0: the tile's first owned cell, at position 4.
+PK_PHYS int fused_end(int T, bool wrap, int c0, int n) { return wrap || c0 + T - 4 <= n + 4 ? T : n + 8 - c0; }
+
+// The roles of position t < end in stage 0 or 1 of the fused sweep: each stage
+// uses up two cells at either end, of the cells that are there.  A circular tile
+// (a whole periodic pencil) has no ends.
+PK_PHYS Roles fused_roles(bool active, bool circ, int t, int end, int stage)
+{
+    const int a = 2 * stage;
+    Roles r;
+    r.end = 0;
+    r.keep = false;
+    r.q = active && (circ || (t >= a && t < end - a));
+    r.slope = active && (circ || (t >= a + 1 && t < end - a - 1));
+    r.flux = active && (circ || (t >= a + 1 && t < end - a - 2));
+    r.upd = active && (circ || (t >= a + 2 && t < end - a - 2));
+    return r;
+}
+
 // Shared-memory planes of a tile, S doubles per plane (S a compile-time bound
 // on the tile's cells, so that every access is one base register plus an
 // immediate offset): Q the primitives, R the right state of each cell's left
@@ -418,9 +440,8 @@ PK_DEV void fused_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
     const int i1 = i1_0 + p;
     const bool circ = tl.circ;
     const int s = circ ? c0 + t : c0 - 4 + t;                  // position along the pencil (interior coords)
-    // a tile that ends beyond the pencil wraps round, or stops at the four guard
-    // cells that the exchange filled: there is nothing of the block behind them
-    const bool active = (tid < PT) && (i1 < g.n1) && (tl.wrap || s < g.n_d + 4);
+    const int end = fused_end(T, circ || tl.wrap, c0, g.n_d);
+    const bool active = (tid < PT) && (i1 < g.n1) && t < end;
     const long long off = (long long)(g.g_d + (tl.wrap ? wrap(s, g.n_d) : s)) * g.sd + (long long)(g.g1 + i1) * g.s1 +
                           (long long)(g.g2 + i2) * g.s2;
     const int mp = circ ? p * pstride + (t == 0 ? T - 1 : t - 1) * st : me - st;
@@ -429,22 +450,15 @@ PK_DEV void fused_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
 #pragma unroll
     for (int v = 0; v < NV; ++v) w[v] = 0.0;
     if (active) load_cell<PH>(uin, off, g, w);
-    Roles r;
-    r.end = 0;
-    r.keep = false;
     const bool own = active && (circ || (t >= 4 && t < T - 4 && s < c0 + tl.L && s < g.n_d));
     FloorRec rec1{0, 0}, rec2{0, 0};
     // both RK2 stages through one copy of the stage code (the solver inlined
     // twice crowds the instruction cache)
 #pragma unroll 1
     for (int stage = 0; stage < 2; ++stage) {
-        // stage 1 (RK2_1) on tile cells [0, T) (circular: every cell); stage 2
-        // (RK2_2) on tile cells [2, T-2), u0 again the sweep's input
-        const int a = 2 * stage;
-        r.q = active && (circ || (t >= a && t < T - a));
-        r.slope = active && (circ || (t >= a + 1 && t < T - a - 1));
-        r.flux = active && (circ || (t >= a + 1 && t < T - a - 2));
-        r.upd = active && (circ || (t >= a + 2 && t < T - a - 2));
+        // stage 1 (RK2_1) on tile cells [0, end) (circular: every cell); stage 2
+        // (RK2_2) on tile cells [2, end-2), u0 again the sweep's input
+        const Roles r = fused_roles(active, circ, t, end, stage);
         FloorRec rec{0, 0};
         rk_stage<PH, S, REC, W3, false, FAST>(smem, me, mp, mn, r, w, uin, uin, off, g, stage == 0 ? dtodx1 : dtodx2, ch,
                                            stp.rch, pp, status, &rec);
