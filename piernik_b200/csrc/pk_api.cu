@@ -939,8 +939,10 @@ int glm_scale(pk_ctx* h, double fac)
 
 // Whether the one-launch sweep with boundary rules serves direction dir of a
 // block that fused_ok refuses: a single gas block, RK2, limited slopes, pencils
-// that fit its CTA, guard cells that hold what the rules say (pk_upload and
-// pk_solve_cg leave others, which the stage path reads as they are).
+// that fit its CTA with their guard cells and are no shorter than the guard
+// width (their images are interior cells), guard cells that hold what the rules
+// say (pk_upload and pk_solve_cg leave others, which the stage path reads as they
+// are).
 bool open_block(pk_ctx* h)
 {
     return !h->connected && h->blocks.size() == 1 && !h->cfg.magnetic && h->cfg.integration_order == 2 &&
@@ -949,7 +951,8 @@ bool open_block(pk_ctx* h)
 
 bool open_ok(pk_ctx* h, int dir)
 {
-    return open_block(h) && h->blocks[0].guards_ruled && h->blocks[0].n[dir] > 1 && h->blocks[0].n[dir] + 4 <= OPEN_T;
+    const Block& b = h->blocks[0];
+    return open_block(h) && b.guards_ruled && b.n[dir] > 1 && b.n[dir] >= b.g[dir] && b.ext[dir] <= OPEN_T;
 }
 
 // sweep(cdim) of all blocks; the step scalars are already in d_step.

@@ -167,6 +167,14 @@ struct OpenCell {
         const double x = Qv[slot];
         return normal && flip ? -x : x;
     }
+    // the state of the cell itself, from that of the interior cell it maps to
+    template <class PH>
+    PK_DEV void mirror(double (&u)[PH::NV]) const
+    {
+#pragma unroll
+        for (int f = 0; f < PH::NFL; ++f)
+            if (fme) u[PH::beg(f) + 1] = -u[PH::beg(f) + 1];
+    }
 };
 
 // The face states of one cell from its own primitives q and its neighbours'
@@ -372,6 +380,7 @@ PK_DEV void rk_stage(double* __restrict__ sm, int me, int mp, int mn, const Role
             for (int v = 0; v < NV; ++v) u0[v] = u0sm[plane_of<PH>(v, perm) * u0st];
         } else {
             load_cell<PH>(u0src, off, g, u0);
+            if constexpr (OPEN) open.mirror<PH>(u0);
         }
 #pragma unroll
         for (int v = 0; v < NV; ++v) w[v] = u0[v] + dtodx * (F[v * S + mp] - (KEEP ? q[v] : F[v * S + me]));
@@ -495,13 +504,20 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sweep_fused(Geom g, Tile tl, con
 
 // -------------------------------------------------------------------------
 // Fused two-stage sweep of one block whose pencils end in outflow, reflecting
-// or periodic rules: P whole pencils per CTA, two cells outside on either side.
-// A cell outside holds no state: where a slope needs its primitives they are
-// those of the interior cell that the rule maps it to, in either stage, as the
-// stage-by-stage sweep finds them in the guard cells that it refreshes between
-// the stages.  Needs guard cells that agree with the rules (the stage path
-// reads whatever they hold).  Against two stage launches and two guard
-// refreshes per sweep: a step of a 149 x 93 x 70 gas box 1.22 -> 0.79 ms.
+// or periodic rules: P whole pencils per CTA, with their guard cells.  A guard
+// cell holds no state of its own: its primitives and its state are those of the
+// interior cell that the rule maps it to, in either stage, as the stage-by-stage
+// sweep finds them in the guard cells that it refreshes between the stages.
+// The interior needs two guard cells on either side; all of them take part
+// because the reference updates a whole pencil and runs the floors over it, ends
+// too: a guard cell that goes negative raises the status, on which a step is
+// redone, although no guard cell is stored here.  (The end cells' floors see
+// the sweep's input in both stages.  The refreshed cells that the stage path
+// gives them in the second are images of stage-1 cells behind their floors:
+// nothing goes negative there that has not raised the status before.)
+// Needs guard cells that agree with the rules (the stage path reads whatever
+// they hold).  Against two stage launches and two guard refreshes per sweep:
+// a step of a 149 x 93 x 70 gas box 1.22 -> 0.82 ms.
 // grid: x = ortho-1 tiles of P pencils, z = ortho-2.
 // -------------------------------------------------------------------------
 template <class PH, int MAXT, int MINB>
@@ -519,9 +535,9 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sweep_open(Geom g, Tile tl, int 
     if (tl.xfast) { t = tid % T; p = tid / T; }
     else { p = tid % P; t = tid / P; }
     const int st = tl.xfast ? 1 : P, me = tid, base = me - t * st;
-    const int i1 = blockIdx.x * P + p, s = t - 2;
+    const int i1 = blockIdx.x * P + p, s = t - g.g_d;
     const bool active = tid < P * T && i1 < g.n1, inner = active && s >= 0 && s < n;
-    // interior cell of position x (-2 .. n + 1) and whether the rule mirrors it
+    // interior cell of position x (-g .. n + g - 1, g <= n) and whether the rule mirrors it
     auto image = [&](int x, bool& flip) {
         flip = false;
         if (x >= 0 && x < n) return x;
@@ -533,17 +549,20 @@ __global__ void __launch_bounds__(MAXT, MINB) k_sweep_open(Geom g, Tile tl, int 
     };
     OpenCell o;
     Roles r;
-    r.end = 0;
-    r.keep = false;
-    r.q = r.upd = inner;
-    r.slope = active && t >= 1 && t <= T - 2;
-    r.flux = active && t >= 1 && t <= T - 3;
-    if (r.slope) {
-        o.me = base + (image(s, o.fme) + 2) * st;
-        o.mp = base + (image(s - 1, o.fmp) + 2) * st;
-        o.mn = base + (image(s + 1, o.fmn) + 2) * st;
+    r.end = t == 0 ? -1 : (t == T - 1 ? 1 : 0);
+    r.q = inner;
+    r.slope = active;
+    r.flux = active && t < T - 1;
+    r.upd = active && r.end == 0;
+    r.keep = active && r.end != 0;
+    int cell = 0;
+    if (active) {                                     // an end cell finds its one neighbour on both sides
+        cell = image(s, o.fme);
+        o.me = base + (cell + g.g_d) * st;
+        o.mp = base + (image(r.end < 0 ? s + 1 : s - 1, o.fmp) + g.g_d) * st;
+        o.mn = base + (image(r.end > 0 ? s - 1 : s + 1, o.fmn) + g.g_d) * st;
     }
-    const long long off = (long long)(g.g_d + (inner ? s : 0)) * g.sd + (long long)(g.g1 + i1) * g.s1 +
+    const long long off = (long long)(g.g_d + cell) * g.sd + (long long)(g.g1 + i1) * g.s1 +
                           (long long)(g.g2 + blockIdx.z) * g.s2;
     double w[NV];
 #pragma unroll

@@ -301,8 +301,8 @@ int launch_fused(pk_ctx* h, Block& b, int dir, int apply_fac)
     return PK_OK;
 }
 
-// The fused sweep of a gas block whose pencils (at most OPEN_T - 4 cells) end in
-// boundary rules
+// The fused sweep of a gas block whose pencils (at most OPEN_T cells with their
+// guard cells) end in boundary rules
 template <class PH>
 int launch_open(pk_ctx* h, Block& b, int dir)
 {
@@ -311,11 +311,11 @@ int launch_open(pk_ctx* h, Block& b, int dir)
     } else {
         Geom g = make_geom(b, dir);
         Tile tl;
-        tl.T = tl.L = b.n[dir] + 4;
+        tl.T = tl.L = b.ext[dir];
         tl.P = OPEN_T / tl.T;
         if (tl.P < 1) return fail(h, PK_E_ARG, "pencil longer than the CTA");
         if (tl.P > g.n1) tl.P = g.n1;
-        tl.halo = 2;
+        tl.halo = b.g[dir];
         tl.xfast = dir == 0;
         dim3 grid((g.n1 + tl.P - 1) / tl.P, 1, g.n2);
         const size_t smem = 3ull * PH::NV * OPEN_T * sizeof(double);

@@ -3,11 +3,14 @@ one-launch sweep (k_sweep_open) against the oracle, bit for bit, guard cells
 included -- short pencils, the longest the CTA holds and one cell more (the
 stage path), every rule on either side, dust beside the gas, guard cells that
 the caller filled differently (the first sweep then reads those, as the
-oracle does), steps replayed from a graph and redone steps."""
+oracle does), steps replayed from a graph and redone steps.  The floors run over
+the guard cells too, as the reference's do: where only one of those goes
+negative the status must say so and a step be redone."""
 import numpy as np
 import pytest
 
 from helpers import assert_bitexact, random_state, setup_for
+from piernik_b200 import problems
 from piernik_b200._lib import PK_RK2_1
 from piernik_b200.config import BND_OUT, BND_PER, BND_REF
 from piernik_b200.sim import Simulation
@@ -80,4 +83,83 @@ def test_open_blocks_options(gpu_lib, oracle_lib, how):
         ob2.run(2)
         gu, _, _ = sim.download()
         assert_bitexact(gu, ob2.u, how + " after a new upload")
+    sim.close()
+
+
+def rough_state(setup, seed, mach):
+    """Densities and pressures over two decades, velocities of either sign."""
+    rng = np.random.default_rng(seed)
+    u, _, _ = problems._empty(setup)
+    shp, g = (setup.n[2], setup.n[1], setup.n[0]), setup.guards
+    rho, p = 10 ** rng.uniform(-1, 1, shp), 10 ** rng.uniform(-1, 1, shp)
+    v = rng.uniform(-mach, mach, shp + (3,))
+    sl = tuple(slice(g[d], g[d] + setup.n[d]) for d in (2, 1, 0))
+    problems._set_fluid(setup, u[sl], 0, rho, v[..., 0], v[..., 1], v[..., 2], p, None)
+    return u
+
+
+# seeds whose first sweep of a 6 x 4 x 5 reflecting box along the axis turns a guard
+# cell negative and no interior one, in stage 1 or 2, found with the oracle
+GUARD_ONLY = [("minmod", 6, 1, 2), ("minmod", 6, 14, 0), ("minmod", 6, 21, 0), ("minmod", 6, 27, 1),
+              ("moncen", 6, 0, 1), ("moncen", 6, 49, 1), ("superbee", 3, 55, 0), ("vanleer", 6, 40, 2)]
+
+
+@pytest.mark.parametrize("lim,mach,seed,axis", GUARD_ONLY + [("minmod", 1, 3, 0), ("moncen", 10, 4, 1)])
+@pytest.mark.parametrize("bnd", [R, O, OR])
+def test_floors_of_guard_cells_raise_the_status(gpu_lib, oracle_lib, lim, mach, seed, axis, bnd):
+    setup = setup_for("hd", n=(6, 4, 5), lim=lim, bnd=(bnd,) * 3)
+    ob = oracle_lib.OracleBlock(setup, rough_state(setup, seed, mach), None, None)
+    ob.fill_guards()
+    sim = Simulation(setup)
+    sim.upload(ob.u)
+    sim.update_boundaries()                # guard cells by the rules: the one-launch sweep
+    dt, _ = ob.timestep_raw()
+    for k in range(2):
+        ob.blk.dn_negative = ob.blk.ei_negative = 0
+        ob.sweep(axis, dt, 0.0)
+        sim.sweep(axis + 1, dt)
+        assert sim.status() == ob.blk.dn_negative + 2 * ob.blk.ei_negative, k
+    gu, _, _ = sim.download()
+    assert_bitexact(gu, ob.u, f"{lim} {seed}")
+    sim.close()
+
+
+@pytest.mark.parametrize("lim,mach,seed,axis", GUARD_ONLY)
+def test_a_negative_guard_cell_redoes_the_step(gpu_lib, oracle_lib, lim, mach, seed, axis):
+    """Sweeps along one axis only, so that the step is redone for nothing else."""
+    setup = setup_for("hd", n=(6, 4, 5), lim=lim, bnd=(R,) * 3, cflcontrol="redo", max_redostep_attempts=30,
+                      skip_sweep=tuple(d != axis for d in range(3)))
+    ob = oracle_lib.OracleBlock(setup, rough_state(setup, seed, mach), None, None)
+    ob.fill_guards()
+    sim = Simulation(setup)
+    sim.upload(ob.u)
+    sim.update_boundaries()
+    for k in range(6):                     # a redone step counts as one of them
+        ob.run(1)
+        sim.run(1)
+        st = sim.time_state
+        assert (st.t, st.dt, st.nstep, st.redone) == (ob.state.t, ob.state.dt, ob.state.nstep, ob.state.redone), k
+    gu, _, _ = sim.download()
+    assert_bitexact(gu, ob.u, f"{lim} {seed}")
+    sim.close()
+
+
+@pytest.mark.parametrize("n,nb", [((248, 5, 4), 4), ((249, 5, 4), 4), ((5, 248, 4), 4), ((250, 6, 6), 3), ((251, 5, 4), 3),
+                                  ((12, 7, 6), 6), ((3, 9, 4), 4), ((2, 8, 2), 2)])
+def test_lengths_at_the_lines_of_the_rule(gpu_lib, oracle_lib, n, nb):
+    """The longest pencil that the CTA holds with its guard cells and one cell
+    more, other guard widths, and pencils shorter than the guard width (both of
+    the latter two go stage by stage)."""
+    setup = setup_for("hd", n=n, lim="moncen", bnd=(R, O, RO), nb=nb)
+    ob = oracle_lib.OracleBlock(setup, random_state(setup, seed=6)[0], None, None)
+    ob.fill_guards()
+    sim = Simulation(setup)
+    sim.upload(ob.u)
+    sim.update_boundaries()
+    for k in range(3):
+        sim.run(1)
+        ob.run(1)
+        gu, _, _ = sim.download()
+        core = tuple(slice(g, g + m) for g, m in zip(setup.guards[::-1], setup.n[::-1]))
+        assert_bitexact(np.ascontiguousarray(gu[core]), np.ascontiguousarray(ob.u[core]), f"{n} step {k}")
     sim.close()
