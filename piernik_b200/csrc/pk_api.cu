@@ -754,7 +754,6 @@ int build_refined_list(pk_ctx* h, int dir, const std::vector<std::vector<StageIt
     }
     if (h->rcount_n < 1 + 2 * nlev) {
         cudaFree(h->d_rcount);
-    cudaFree(h->d_eglm);
         h->d_rcount = nullptr;
         h->rcount_n = 1 + 2 * nlev;
         PK_CUDA(h, cudaMalloc(&h->d_rcount, sizeof(unsigned) * h->rcount_n));

@@ -94,3 +94,53 @@ def test_eglm_rejections(gpu_lib):
     with pytest.raises(PkError, match="E-GLM"):
         sim.grad_forward(1, 1)
     sim.close()
+
+
+def test_eglm_after_a_refused_refined_step(gpu_lib):
+    """E-GLM does not run on refined domains: a step with a refined block is
+    refused, after the sweeps' work lists were built.  Without that block the
+    domain must run on as if it had never been there (the E-GLM scratch memory
+    is the handle's for as long as it lives)."""
+    from test_gpu_blocks import exact_dl, tiles, window
+    full = exact_dl(setup_for("mhd", n=(32, 16, 16), lim="moncen", use_eglm=True))
+    state = random_state(full, seed=10)
+
+    def domain():
+        sim = None
+        for n, off in tiles([16, 16], [16], [16]):
+            s = full.replace(n=n, xmin=tuple(o * d for o, d in zip(off, full.dl)),
+                             xmax=tuple((o + m) * d for o, m, d in zip(off, n, full.dl)))
+            if sim is None:
+                sim, bid = Simulation(s), 0
+                sim.set_domain(full.n, (True, True, True))
+            else:
+                bid = sim.add_block(s)
+            sim.place_block(bid, off)
+            sim.upload(*(window(full, x, n, off) for x in state), block=bid)
+        sim.update_boundaries()
+        sim.run(1)
+        return sim
+
+    def resume(sim, kept, st):
+        for i, arrs in enumerate(kept):
+            sim.upload(*arrs, block=i)
+        sim.time_state = st
+        sim.update_boundaries()
+        sim.run(2)
+        out = [sim.download(block=i) for i in range(2)]
+        sim.close()
+        return out
+
+    sim, other = domain(), domain()
+    st, kept = sim.time_state, [sim.download(block=i) for i in range(2)]
+    fine = full.replace(n=(8, 8, 8), xmin=(0.25,) * 3, xmax=tuple(0.25 + 8 * d / 2 for d in full.dl))
+    k = sim.add_block(fine)
+    sim.place_block(k, (8, 8, 8), 1)
+    sim.prolong_block(k)
+    sim.update_boundaries()
+    with pytest.raises(PkError, match="eglm"):
+        sim.run(1)
+    sim.remove_block(k)
+    for got, want in zip(resume(sim, kept, st), resume(other, kept, st)):
+        for a, w, name in zip(got, want, ("u", "b", "psi")):
+            assert_bitexact(a, w, name)
