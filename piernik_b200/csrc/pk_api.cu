@@ -869,10 +869,12 @@ int build_batch(pk_ctx* h)
 
 void invalidate_graph(pk_ctx* h)
 {
-    if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);
-    if (h->graph) cudaGraphDestroy(h->graph);
-    h->graph_exec = nullptr;
-    h->graph = nullptr;
+    for (auto& sg : h->step_graph) {
+        if (sg.exec) cudaGraphExecDestroy(sg.exec);
+        if (sg.graph) cudaGraphDestroy(sg.graph);
+        sg.exec = nullptr;
+        sg.graph = nullptr;
+    }
 }
 
 int put_step_params(pk_ctx* h, double dt, double ch, double fac)
@@ -1967,10 +1969,9 @@ static int run_step_sweeps(pk_ctx* h, double dt, double ch, double fac)
         for (auto& b : h->blocks)
             if (!b.uh && !fused_ok(h)) PK_CUDA(h, cudaMalloc(&b.uh, sizeof(double) * h->nplanes * b.plane));
         if (int rc = eglm_alloc(h)) return rc;
-        if (h->graph_exec && h->graph_cur != h->cur) invalidate_graph(h);   // it reads the other parity's buffer
-        if (!h->graph_exec) {
-            h->graph_cur = h->cur;
-            // capture the sweeps of one step once; the step scalars are read from d_step
+        pk_ctx::StepGraph& sg = h->step_graph[h->cur];
+        if (!sg.exec) {
+            // capture the sweeps of one step once per parity; the step scalars are read from d_step
             const int cur0 = h->cur;
             const long long l0 = h->launches;
             PK_CUDA(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
@@ -1978,10 +1979,10 @@ static int run_step_sweeps(pk_ctx* h, double dt, double ch, double fac)
             if (open_block(h)) h->blocks[0].guards_stale = true;   // the captured step refreshes what its stages read
             const int rc = step_sweeps(h, dt, ch, fac);
             if (open_block(h)) {
-                h->graph_stale = h->blocks[0].guards_stale;
+                sg.stale = h->blocks[0].guards_stale;
                 h->blocks[0].guards_stale = stale0;
             }
-            h->graph_kernels = h->launches - l0;
+            sg.kernels = h->launches - l0;
             h->launches = l0;                 // counted when the graph is launched
             cudaGraph_t g = nullptr;
             const cudaError_t e = cudaStreamEndCapture(h->stream, &g);
@@ -1991,15 +1992,15 @@ static int run_step_sweeps(pk_ctx* h, double dt, double ch, double fac)
                 return rc;
             }
             if (e != cudaSuccess) return fail(h, PK_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-            h->graph = g;
-            PK_CUDA(h, cudaGraphInstantiate(&h->graph_exec, g, 0));
+            sg.graph = g;
+            PK_CUDA(h, cudaGraphInstantiate(&sg.exec, g, 0));
         }
-        PK_CUDA(h, cudaGraphLaunch(h->graph_exec, h->stream));
-        h->launches += h->graph_kernels;
+        PK_CUDA(h, cudaGraphLaunch(sg.exec, h->stream));
+        h->launches += sg.kernels;
         if (fused_ok(h))
             for (auto& b : h->blocks) b.guards_stale = true;
         else if (open_block(h))
-            h->blocks[0].guards_stale = h->graph_stale;
+            h->blocks[0].guards_stale = sg.stale;
         return PK_OK;
     }
     return step_sweeps(h, dt, ch, fac);

@@ -160,12 +160,18 @@ struct pk_ctx {
     long long launches = 0;             // kernels of this library launched on the handle's stream
     bool profiling = false;             // bracket sweep kernels with CUDA events
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev_used, ev_free;
-    cudaGraph_t graph = nullptr;        // captured sweeps of one step (pk_run with graphs)
-    cudaGraphExec_t graph_exec = nullptr;
+    // the sweeps of one step captured once (pk_run with graphs), one graph per
+    // parity of the state that it reads: a step's sweeps swap the buffers an even
+    // number of times, but a step launched one by one after an upload or single
+    // sweeps (pk_sweep) may leave the other parity
+    struct StepGraph {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        long long kernels = 0;          // kernel nodes of the captured step
+        bool stale = false;             // the step of a block with boundary rules leaves its guards stale
+    };
+    StepGraph step_graph[2];
     int use_graph = 0;
-    long long graph_kernels = 0;        // kernel nodes of the captured step
-    int graph_cur = 0;                  // the parity whose state the captured step reads
-    bool graph_stale = false;           // the captured step of a block with boundary rules leaves its guards stale
     // same-level domain of connected blocks (pk_set_domain / pk_block_place)
     bool connected = false;
     long long dom[3] = {1, 1, 1};

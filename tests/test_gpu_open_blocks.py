@@ -163,3 +163,33 @@ def test_lengths_at_the_lines_of_the_rule(gpu_lib, oracle_lib, n, nb):
         core = tuple(slice(g, g + m) for g, m in zip(setup.guards[::-1], setup.n[::-1]))
         assert_bitexact(np.ascontiguousarray(gu[core]), np.ascontiguousarray(ob.u[core]), f"{n} step {k}")
     sim.close()
+
+
+@pytest.mark.parametrize("phys,bnd", [("hd", (OR, R, O)), ("hd", (P, P, P)), ("mhd", (P, P, P))])
+def test_graphs_of_either_parity(gpu_lib, phys, bnd):
+    """A captured step reads one of the two state buffers.  Single sweeps and the
+    step that follows an upload (launched one by one for an open block) leave the
+    state in the other: steps replayed in any order of the two must equal steps
+    launched one by one."""
+    setup = setup_for(phys, n=(24, 18, 14), lim="moncen", bnd=bnd)
+    state = random_state(setup, seed=7)
+    sims = [Simulation(setup), Simulation(setup)]
+    sims[1].use_graph()
+    start = sims[0].time_state
+    for sim in sims:
+        for what in ("upload", "run", "run", "sweep", "run", "upload", "run", "run", "sweep", "sweep", "run", "upload", "run",
+                     "run"):
+            if what == "upload":
+                sim.upload(*state)
+                sim.time_state = start
+            elif what == "sweep":
+                sim.sweep(2, 1e-3, 1.0)
+            else:
+                sim.run(2)
+    (u, b, psi), (gu, gb, gp) = (sim.download() for sim in sims)
+    assert_bitexact(gu, u, "u")
+    if setup.magnetic:
+        assert_bitexact(gb, b, "b")
+        assert_bitexact(gp, psi, "psi")
+    for sim in sims:
+        sim.close()
