@@ -206,22 +206,30 @@ PK_PHYS double half_slope(double dl, double dr)
 // WENO3 face states of cell c from q(c-1), q(c), q(c+1) (interpolations.F90:
 // 210-337, Yamaleev & Carpenter 2009): ql = the left state of the right face,
 // qr = the right state of the left face, in the reference's operation order.
-PK_PHYS void weno3_faces(double qm, double qc, double qp, double weps, double& ql, double& qr)
+// Six quotients a component by four denominators (tau / (weps + b) serves both
+// faces): an arithmetic A of the policies above.
+template <class A>
+PK_PHYS void weno3_faces(A& ar, double qm, double qc, double qp, double weps, double& ql, double& qr)
 {
     const double d0 = 2.0 / 3.0, d1 = 1.0 / 3.0;                              // Eq. 19 (twot, onet)
     const double b0 = (qp - qc) * (qp - qc);                                    // Eq. 20
     const double b1 = (qc - qm) * (qc - qm);
     const double tt = ((qp - 2.0 * qc) + qm);                                   // Eq. 22
     const double tau = tt * tt;
-    double a0 = d0 * (1.0 + tau / (weps + b0));                                 // Eq. 21
-    double a1 = d1 * (1.0 + tau / (weps + b1));
-    double w0 = a0 / (a0 + a1), w1 = a1 / (a0 + a1);                            // Eq. 18
+    const double e0 = weps + b0, e1 = weps + b1;
+    const double t0 = ar.quoz(tau, e0, ar.inv(e0)), t1 = ar.quoz(tau, e1, ar.inv(e1));
+    double a0 = d0 * (1.0 + t0);                                                // Eq. 21
+    double a1 = d1 * (1.0 + t1);
+    double s = a0 + a1, r = ar.inv(s);
+    double w0 = ar.quo(a0, s, r), w1 = ar.quo(a1, s, r);                        // Eq. 18
     double f0 = 0.5 * (qc + qp), f1 = 0.5 * (-qm + 3.0 * qc);                   // Eq. 15
     ql = w0 * f0 + w1 * f1;                                                     // Eq. 14
-    a0 = d0 * (1.0 + tau / (weps + b1));                                        // the mirrored stencil
-    a1 = d1 * (1.0 + tau / (weps + b0));
-    w0 = a0 / (a0 + a1);
-    w1 = a1 / (a0 + a1);
+    a0 = d0 * (1.0 + t1);                                                       // the mirrored stencil
+    a1 = d1 * (1.0 + t0);
+    s = a0 + a1;
+    r = ar.inv(s);
+    w0 = ar.quo(a0, s, r);
+    w1 = ar.quo(a1, s, r);
     f0 = 0.5 * (qc + qm);
     f1 = 0.5 * (-qp + 3.0 * qc);
     qr = w0 * f0 + w1 * f1;

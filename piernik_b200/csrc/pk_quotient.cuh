@@ -130,6 +130,12 @@ static __device__ __noinline__ void hllc_ieee(bool has_energy, double gamma, con
     hllc_iface(has_energy, gamma, x, x + 5, f);
 }
 
+static __device__ __noinline__ void weno3_ieee(double qm, double qc, double qp, double weps, double* lr)
+{
+    Ieee ar;
+    weno3_faces(ar, qm, qc, qp, weps, lr[0], lr[1]);
+}
+
 static __device__ __noinline__ double divide_ieee(double n, double d) { return n / d; }
 
 // n / d, correctly rounded: the floors' quotient
