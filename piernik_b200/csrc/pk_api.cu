@@ -107,6 +107,9 @@ const PhysOps* ops_of(pk_ctx* h)
     }
 }
 
+// the recording and adjoint sweeps (null: not built for these fluids)
+const GradOps* grad_ops_of(pk_ctx* h) { return h->phys == 0 ? grad_ops_hd1() : (h->phys == 2 ? grad_ops_mhd1() : nullptr); }
+
 BoxGeom box_of(const Block& b)
 {
     BoxGeom bg;
@@ -1954,6 +1957,21 @@ static int clamp_dt(const pk_config& c, pk_time_state& ts, double dt, double c_a
     return PK_OK;
 }
 
+// the kernels that a lone block's sweeps load at their first use, before a capture
+static int ready_step(pk_ctx* h)
+{
+    if (!fused_ok(h)) return open_block(h) ? ops_of(h)->ready_open(h) : PK_OK;
+    if (h->blocks.size() != 1 || (h->batched && h->ninst < 2)) return PK_OK;
+    int dirs[3], nd;
+    step_dirs(h, dirs, &nd);
+    for (int s = 0; s < nd; ++s) {
+        const int rc = h->arith == PK_ARITH_FMA ? fast_ops_of(h)->ready(h, h->blocks[0], dirs[s])
+                                                : ops_of(h)->ready(h, h->blocks[0], dirs[s]);
+        if (rc) return rc;
+    }
+    return PK_OK;
+}
+
 // the sweeps of one step, the step scalars already in d_step: replayed from a
 // CUDA graph captured once (use_graph) or launched one by one
 static int run_step_sweeps(pk_ctx* h, double dt, double ch, double fac)
@@ -1971,6 +1989,7 @@ static int run_step_sweeps(pk_ctx* h, double dt, double ch, double fac)
         if (int rc = eglm_alloc(h)) return rc;
         pk_ctx::StepGraph& sg = h->step_graph[h->cur];
         if (!sg.exec) {
+            if (int rc = ready_step(h)) return rc;
             // capture the sweeps of one step once per parity; the step scalars are read from d_step
             const int cur0 = h->cur;
             const long long l0 = h->launches;
@@ -2512,7 +2531,8 @@ int grad_check(pk_ctx* h)
     if (h->blocks.size() != 1 || !h->remote.empty())
         return fail(h, PK_E_UNSUPPORTED, "the differentiable path runs on one block of one rank");
     if (!fused_ok(h)) return fail(h, PK_E_UNSUPPORTED, "the differentiable path needs RK2 and periodic boundaries");
-    if (h->cfg.nfluids != 1) return fail(h, PK_E_UNSUPPORTED, "the differentiable path is built for one fluid");
+    if (h->cfg.nfluids != 1 || !grad_ops_of(h))
+        return fail(h, PK_E_UNSUPPORTED, "the differentiable path is built for one fluid");
     if (h->cfg.use_eglm) return fail(h, PK_E_UNSUPPORTED, "the differentiable path has no E-GLM sources");
     if (h->cfg.interpolation != PK_INTERP_LINEAR)
         return fail(h, PK_E_UNSUPPORTED, "the differentiable path differentiates the linear (limited) reconstruction");
@@ -2629,7 +2649,7 @@ int pk_adjoint_sweep(pk_handle h, int32_t cdim, double dt, double chspeed)
     if (int rc = grad_check(h)) return rc;
     if (!h->lam) return fail(h, PK_E_STATE, "set the adjoint first (pk_adjoint_set)");
     Block& b = h->blocks[0];
-    const PhysOps* ops = ops_of(h);
+    const GradOps* ops = grad_ops_of(h);
     if (int rc = ensure_pool(h, b, 1)) return rc;
     if (int rc = put_step_params(h, dt, chspeed, 1.0)) return rc;
     const int d = cdim - 1;
@@ -2707,7 +2727,7 @@ int pk_grad_backward(pk_handle h)
     if (int rc = grad_check(h)) return rc;
     if (!h->lam) return fail(h, PK_E_STATE, "set the adjoint of the final state first (pk_adjoint_set)");
     Block& b = h->blocks[0];
-    const PhysOps* ops = ops_of(h);
+    const GradOps* ops = grad_ops_of(h);
     int dir[6], fac[6];
     const int nsw = step_plan(h, dir, fac);
     const int ni = h->ninst;

@@ -257,6 +257,8 @@ Geom make_geom(const Block& b, int dir);
 struct PhysOps {
     int nv;
     int (*prepare)(pk_ctx* h);      // kernel attributes; called before any launch or graph capture
+    int (*ready)(pk_ctx* h, Block& b, int dir);     // the same of a lone block's staged kernel along dir, before a capture
+    int (*ready_open)(pk_ctx* h);                   // ... of the sweep with boundary rules
     int (*fused)(pk_ctx* h, Block& b, int dir, int apply_fac);
     int (*open)(pk_ctx* h, Block& b, int dir);      // a sweep of pencils with boundary rules (gas only)
     int (*stage)(pk_ctx* h, Block& b, int dir, int first, double rk);           // dt, ch from d_step
@@ -264,18 +266,24 @@ struct PhysOps {
     int (*stage_refined)(pk_ctx* h, int dir, int first, double rk);             // all levels, one launch
     int (*batched)(pk_ctx* h, int dir, int apply_fac, unsigned* counter);
     int (*fused_ptr)(pk_ctx* h, Block& b, int dir, int apply_fac, const double* in, double* out);
+    int (*unsplit_flux)(pk_ctx* h, Block& b, int dir, const double* in, double* F);
+    int (*unsplit_apply)(pk_ctx* h, Block& b, const double* S, double* T, double rk, int last);
+};
+
+// the differentiable path's sweeps (pk_grad_*.cu, one fluid): units of their own,
+// so that the device code that a forward run's first handle loads is without them
+struct GradOps {
     int (*fused_rec)(pk_ctx* h, Block& b, int dir, int apply_fac, const double* in, double* out, double* ustar,
                      unsigned short* flags);
     int (*adj)(pk_ctx* h, Block& b, int dir, int apply_fac, const double* uin, const double* ustar,
                const double* uout, const unsigned short* flags, const double* lam_out, double* lam_in, double* m1);
-    int (*unsplit_flux)(pk_ctx* h, Block& b, int dir, const double* in, double* F);
-    int (*unsplit_apply)(pk_ctx* h, Block& b, const double* S, double* T, double rk, int last);
 };
 
 // the fused and batched sweeps in the tolerance-mode arithmetic (pk_fast_*.cu,
 // compiled with multiply-add contraction; pk_set_arithmetic)
 struct FastOps {
     int (*prepare)(pk_ctx* h);
+    int (*ready)(pk_ctx* h, Block& b, int dir);
     int (*fused)(pk_ctx* h, Block& b, int dir, int apply_fac);
     int (*batched)(pk_ctx* h, int dir, int apply_fac, unsigned* counter);
 };
@@ -285,6 +293,9 @@ const FastOps* fast_ops_hd2();
 const FastOps* fast_ops_mhd1();
 const FastOps* fast_ops_mhd2();
 const FastOps* fast_ops_mhd3();
+
+const GradOps* grad_ops_hd1();
+const GradOps* grad_ops_mhd1();
 
 const PhysOps* ops_hd1();
 const PhysOps* ops_hd2();

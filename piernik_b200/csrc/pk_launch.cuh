@@ -80,10 +80,38 @@ int set_fused_attr(pk_ctx* h)
                                         220 * 1024));
         PK_CUDA(h, cudaFuncSetAttribute(batched_variant<PH, FAST>(0, true),
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-        for (int n : {64, 128, 256})
-            PK_CUDA(h, cudaFuncSetAttribute(staged_kernel<PH, FAST>(n), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            220 * 1024));
         done = true;
+    }
+    return PK_OK;
+}
+
+// the same for one kernel at its first use: setting the limit loads the kernel,
+// and a process should not pay with its first handle for kernels that it does not
+// run (the three staged kernels, the sweep with boundary rules, the adjoint's)
+template <class F>
+int raise_smem(pk_ctx* h, F* kernel, bool* done)
+{
+    if (!*done)
+        PK_CUDA(h, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    *done = true;
+    return PK_OK;
+}
+
+// ... the staged kernel of pencils of n cells
+template <class PH, bool FAST, bool REC>
+int set_staged_attr(pk_ctx* h, int n)
+{
+    static bool done[3] = {};
+    const int S = staged_stride(n);
+    return raise_smem(h, staged_kernel<PH, FAST, REC>(n), done + (S == 64 ? 0 : (S == 128 ? 1 : 2)));
+}
+
+template <class PH>
+int set_open_attr(pk_ctx* h)
+{
+    if constexpr (!PH::MHD) {
+        static bool done = false;
+        return raise_smem(h, k_sweep_open<PH, OPEN_T, 2>, &done);
     }
     return PK_OK;
 }
@@ -121,9 +149,6 @@ int set_smem_attr(pk_ctx* h)
     static bool done = false;
     if (!done) {
         if (int rc = set_fused_attr<PH, false>(h)) return rc;
-        if constexpr (!PH::MHD)
-            PK_CUDA(h, cudaFuncSetAttribute(k_sweep_open<PH, OPEN_T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            220 * 1024));
         PK_CUDA(h, cudaFuncSetAttribute(k_stage<PH, STAGE_MAXT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         PK_CUDA(h, cudaFuncSetAttribute(k_stage<PH, STAGE_MAXT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         220 * 1024));
@@ -276,6 +301,7 @@ int launch_fused_ptr(pk_ctx* h, Block& b, int dir, int apply_fac, const double* 
         if (!encode_state_map(&tin, in, b.n, b.ext, b.plane, PH::NV, dir) ||
             !encode_state_map(&tout, out, b.n, b.ext, b.plane, PH::NV, dir))
             return fail(h, PK_E_CUDA, "cuTensorMapEncodeTiled failed for the staged sweep");
+        if (int rc = set_staged_attr<PH, FAST, false>(h, b.n[dir])) return rc;
         const int threads = (b.n[dir] + 31) / 32 * 32;
         if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
         staged_kernel<PH, FAST>(b.n[dir])<<<grid, threads, staged_smem(PH::NV, b.n[dir]), h->stream>>>(
@@ -301,6 +327,20 @@ int launch_fused(pk_ctx* h, Block& b, int dir, int apply_fac)
     return PK_OK;
 }
 
+// the kernels with a limit of their own that the sweeps of a lone block along dir
+// will launch, loaded before a step is captured
+template <class PH, bool FAST = false>
+int ready_sweep(pk_ctx* h, Block& b, int dir)
+{
+    if (b.n[dir] <= 1) return PK_OK;
+    Geom g = make_geom(b, dir);
+    Tile tl;
+    dim3 grid;
+    int var;
+    if (int rc = fused_geometry(h, b, dir, g, &tl, &grid, &var, !h->pp.weno3)) return rc;
+    return var == VAR_STAGED ? set_staged_attr<PH, FAST, false>(h, b.n[dir]) : PK_OK;
+}
+
 // The fused sweep of a gas block whose pencils (at most OPEN_T cells with their
 // guard cells) end in boundary rules
 template <class PH>
@@ -314,6 +354,7 @@ int launch_open(pk_ctx* h, Block& b, int dir)
         tl.T = tl.L = b.ext[dir];
         tl.P = OPEN_T / tl.T;
         if (tl.P < 1) return fail(h, PK_E_ARG, "pencil longer than the CTA");
+        if (int rc = set_open_attr<PH>(h)) return rc;
         if (tl.P > g.n1) tl.P = g.n1;
         tl.halo = b.g[dir];
         tl.xfast = dir == 0;
@@ -358,45 +399,35 @@ template <class PH>
 int launch_fused_rec(pk_ctx* h, Block& b, int dir, int apply_fac, const double* in, double* out, double* ustar,
                      unsigned short* flags)
 {
-    if constexpr (PH::NFL != 1) {
-        return fail(h, PK_E_UNSUPPORTED, "the differentiable path is built for one-fluid HD and MHD");
+    static_assert(PH::NFL == 1, "the differentiable path is built for one fluid");
+    Geom g = make_geom(b, dir);
+    Tile tl;
+    dim3 grid;
+    int var;
+    if (int rc = fused_geometry(h, b, dir, g, &tl, &grid, &var, true)) return rc;
+    std::pair<cudaEvent_t, cudaEvent_t> ev;
+    if (var == VAR_STAGED) {
+        CUtensorMap tin, tout;
+        if (!encode_state_map(&tin, in, b.n, b.ext, b.plane, PH::NV, dir) ||
+            !encode_state_map(&tout, out, b.n, b.ext, b.plane, PH::NV, dir))
+            return fail(h, PK_E_CUDA, "cuTensorMapEncodeTiled failed for the staged sweep");
+        if (int rc = set_staged_attr<PH, false, true>(h, b.n[dir])) return rc;
+        const int threads = (b.n[dir] + 31) / 32 * 32;
+        if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
+        staged_kernel<PH, false, true>(b.n[dir])<<<grid, threads, staged_smem(PH::NV, b.n[dir]), h->stream>>>(
+            tin, tout, g, h->pp, b.dl[dir], h->d_step, apply_fac, dir, h->d_status, ustar, flags);
     } else {
-        static bool attr = false;
-        if (!attr) {
-            for (int v = 0; v < NVARIANT; ++v)
-                PK_CUDA(h, cudaFuncSetAttribute(rec_variant<PH>(v), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                220 * 1024));
-            for (int n : {64, 128, 256})
-                PK_CUDA(h, cudaFuncSetAttribute(staged_kernel<PH, false, true>(n),
-                                                cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-            attr = true;
-        }
-        Geom g = make_geom(b, dir);
-        Tile tl;
-        dim3 grid;
-        int var;
-        if (int rc = fused_geometry(h, b, dir, g, &tl, &grid, &var, true)) return rc;
-        std::pair<cudaEvent_t, cudaEvent_t> ev;
-        if (var == VAR_STAGED) {
-            CUtensorMap tin, tout;
-            if (!encode_state_map(&tin, in, b.n, b.ext, b.plane, PH::NV, dir) ||
-                !encode_state_map(&tout, out, b.n, b.ext, b.plane, PH::NV, dir))
-                return fail(h, PK_E_CUDA, "cuTensorMapEncodeTiled failed for the staged sweep");
-            const int threads = (b.n[dir] + 31) / 32 * 32;
-            if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
-            staged_kernel<PH, false, true>(b.n[dir])<<<grid, threads, staged_smem(PH::NV, b.n[dir]), h->stream>>>(
-                tin, tout, g, h->pp, b.dl[dir], h->d_step, apply_fac, dir, h->d_status, ustar, flags);
-        } else {
-            const size_t smem = 3ull * PH::NV * VAR_T[var] * sizeof(double);
-            if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
-            rec_variant<PH>(var)<<<grid, tl.P * tl.T, smem, h->stream>>>(g, tl, in, out, ustar, flags, h->pp,
-                                                                        b.dl[dir], h->d_step, apply_fac, h->d_status);
-        }
-        PK_CUDA(h, cudaGetLastError());
-        if (int rc = ev_end(h, ev)) return fail(h, rc, "cudaEventRecord failed");
-        h->launches += 1;
-        return PK_OK;
+        const size_t smem = 3ull * PH::NV * VAR_T[var] * sizeof(double);
+        static bool done[NVARIANT] = {};
+        if (int rc = raise_smem(h, rec_variant<PH>(var), done + var)) return rc;
+        if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
+        rec_variant<PH>(var)<<<grid, tl.P * tl.T, smem, h->stream>>>(g, tl, in, out, ustar, flags, h->pp,
+                                                                    b.dl[dir], h->d_step, apply_fac, h->d_status);
     }
+    PK_CUDA(h, cudaGetLastError());
+    if (int rc = ev_end(h, ev)) return fail(h, rc, "cudaEventRecord failed");
+    h->launches += 1;
+    return PK_OK;
 }
 
 // Launch-bound variants of the two adjoint kernels (threads per CTA, CTAs per
@@ -453,96 +484,88 @@ template <class PH>
 int launch_adj(pk_ctx* h, Block& b, int dir, int apply_fac, const double* uin, const double* ustar, const double* uout,
                const unsigned short* flags, const double* lam_out, double* lam_in, double* m1)
 {
-    if constexpr (PH::NFL != 1) {
-        return fail(h, PK_E_UNSUPPORTED, "the adjoint sweep is built for one-fluid HD and MHD");
-    } else {
-        static bool attr = false;
-        if (!attr) {
-            for (int v = 0; v < ADJ_VAR_STAGED; ++v) {
-                const AdjKernels<PH> k = adj_variant<PH>(v);
-                PK_CUDA(h, cudaFuncSetAttribute(k.s2, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-                PK_CUDA(h, cudaFuncSetAttribute(k.s1, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    static_assert(PH::NFL == 1, "the differentiable path is built for one fluid");
+    int var = (h->adjV[dir] >= 0 && h->adjV[dir] < NADJ_VARIANT) ? h->adjV[dir] : DEF_ADJ_V[dir];
+    Geom g = make_geom(b, dir);
+    if (var == ADJ_VAR_STAGED) {
+        if (staged_ok(b.n, b.g, b.ext, h->nplanes, dir, g.seg_len)) {
+            CUtensorMap m_ustar, m_lamout, m_lamin, m_m1, m_uin;
+            if (!encode_state_map(&m_ustar, ustar, b.n, b.ext, b.plane, PH::NV, dir) ||
+                !encode_state_map(&m_lamout, lam_out, b.n, b.ext, b.plane, PH::NV, dir) ||
+                !encode_state_map(&m_lamin, lam_in, b.n, b.ext, b.plane, PH::NV, dir) ||
+                !encode_state_map(&m_m1, m1, b.n, b.ext, b.plane, PH::NV, dir) ||
+                !encode_state_map(&m_uin, uin, b.n, b.ext, b.plane, PH::NV, dir))
+                return fail(h, PK_E_CUDA, "cuTensorMapEncodeTiled failed for the staged adjoint sweep");
+            static bool done[3] = {};
+            if (int rc = raise_smem(h, k_adj_staged2<PH>, done)) return rc;
+            if (int rc = raise_smem(h, k_adj_staged1<PH>, done + 1)) return rc;
+            if (dir != 0)
+                if (int rc = raise_smem(h, k_adj_staged1_boxed<PH>, done + 2)) return rc;
+            const int threads = (b.n[dir] + 31) / 32 * 32;
+            // persistent: as many CTAs as can be resident (one per SM at
+            // 256 threads, more for shorter pencils), over the tiles (pairs of pencils)
+            const long long ntiles = (long long)((g.n1 + 1) / 2) * g.n2;
+            const size_t smem = adj_staged_smem(PH::NV, b.n[dir]);
+            int per_sm = 0;
+            PK_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                           &per_sm, dir == 0 ? (const void*)k_adj_staged1<PH> : (const void*)k_adj_staged2<PH>,
+                           threads, smem));
+            if (per_sm < 1) per_sm = 1;
+            const int ctas = (int)std::min<long long>(ntiles, (long long)per_sm * sm_count());
+            std::pair<cudaEvent_t, cudaEvent_t> ev;
+            if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
+            k_adj_staged2<PH><<<ctas, threads, smem, h->stream>>>(m_ustar, m_lamout, m_lamin, m_m1, g, uout,
+                                                                  flags, h->pp, b.dl[dir], h->d_step,
+                                                                  apply_fac, dir, h->d_status);
+            PK_CUDA(h, cudaGetLastError());
+            if (dir == 0) {
+                k_adj_staged1<PH><<<ctas, threads, smem, h->stream>>>(m_uin, m_m1, g, lam_in, h->pp, h->d_step,
+                                                                      dir, h->d_status);
+            } else {
+                const dim3 grid((g.n1 + 1) / 2, 1, g.n2);
+                k_adj_staged1_boxed<PH><<<grid, threads, adj_staged1_boxed_smem(PH::NV, b.n[dir]), h->stream>>>(
+                    m_uin, m_m1, m_lamin, g, h->pp, h->d_step, dir, h->d_status);
             }
-            PK_CUDA(h, cudaFuncSetAttribute(k_adj_staged2<PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-            PK_CUDA(h, cudaFuncSetAttribute(k_adj_staged1<PH>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-            PK_CUDA(h, cudaFuncSetAttribute(k_adj_staged1_boxed<PH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            220 * 1024));
-            attr = true;
+            PK_CUDA(h, cudaGetLastError());
+            if (int rc = ev_end(h, ev)) return fail(h, rc, "cudaEventRecord failed");
+            h->launches += 2;
+            return PK_OK;
         }
-        int var = (h->adjV[dir] >= 0 && h->adjV[dir] < NADJ_VARIANT) ? h->adjV[dir] : DEF_ADJ_V[dir];
-        Geom g = make_geom(b, dir);
-        if (var == ADJ_VAR_STAGED) {
-            if (staged_ok(b.n, b.g, b.ext, h->nplanes, dir, g.seg_len)) {
-                CUtensorMap m_ustar, m_lamout, m_lamin, m_m1, m_uin;
-                if (!encode_state_map(&m_ustar, ustar, b.n, b.ext, b.plane, PH::NV, dir) ||
-                    !encode_state_map(&m_lamout, lam_out, b.n, b.ext, b.plane, PH::NV, dir) ||
-                    !encode_state_map(&m_lamin, lam_in, b.n, b.ext, b.plane, PH::NV, dir) ||
-                    !encode_state_map(&m_m1, m1, b.n, b.ext, b.plane, PH::NV, dir) ||
-                    !encode_state_map(&m_uin, uin, b.n, b.ext, b.plane, PH::NV, dir))
-                    return fail(h, PK_E_CUDA, "cuTensorMapEncodeTiled failed for the staged adjoint sweep");
-                const int threads = (b.n[dir] + 31) / 32 * 32;
-                // persistent: as many CTAs as can be resident (one per SM at
-                // 256 threads, more for shorter pencils), over the tiles (pairs of pencils)
-                const long long ntiles = (long long)((g.n1 + 1) / 2) * g.n2;
-                const size_t smem = adj_staged_smem(PH::NV, b.n[dir]);
-                int per_sm = 0;
-                PK_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                               &per_sm, dir == 0 ? (const void*)k_adj_staged1<PH> : (const void*)k_adj_staged2<PH>,
-                               threads, smem));
-                if (per_sm < 1) per_sm = 1;
-                const int ctas = (int)std::min<long long>(ntiles, (long long)per_sm * sm_count());
-                std::pair<cudaEvent_t, cudaEvent_t> ev;
-                if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
-                k_adj_staged2<PH><<<ctas, threads, smem, h->stream>>>(m_ustar, m_lamout, m_lamin, m_m1, g, uout,
-                                                                      flags, h->pp, b.dl[dir], h->d_step,
-                                                                      apply_fac, dir, h->d_status);
-                PK_CUDA(h, cudaGetLastError());
-                if (dir == 0) {
-                    k_adj_staged1<PH><<<ctas, threads, smem, h->stream>>>(m_uin, m_m1, g, lam_in, h->pp, h->d_step,
-                                                                          dir, h->d_status);
-                } else {
-                    const dim3 grid((g.n1 + 1) / 2, 1, g.n2);
-                    k_adj_staged1_boxed<PH><<<grid, threads, adj_staged1_boxed_smem(PH::NV, b.n[dir]), h->stream>>>(
-                        m_uin, m_m1, m_lamin, g, h->pp, h->d_step, dir, h->d_status);
-                }
-                PK_CUDA(h, cudaGetLastError());
-                if (int rc = ev_end(h, ev)) return fail(h, rc, "cudaEventRecord failed");
-                h->launches += 2;
-                return PK_OK;
-            }
-            var = 0;                                  // not stageable here: the tiled default
-        }
-        Tile tl;
-        int L = h->adjL[dir] > 0 ? h->adjL[dir] : default_adj_length(dir, b.n[dir], ADJ_T[var]);
-        if (L > b.n[dir]) L = b.n[dir];
-        tl.circ = (L == b.n[dir] && b.n[dir] <= ADJ_T[var]) ? 1 : 0;
-        if (g.seg_len && g.seg_along) {               // stacked instances: one whole segment per tile
-            L = g.seg_len;
-            tl.circ = 1;
-            if (L > ADJ_T[var]) return fail(h, PK_E_ARG, "instance segment longer than the adjoint variant's CTA size");
-        }
-        if (!tl.circ && L > ADJ_T[var] - 6) L = ADJ_T[var] - 6;
-        tl.T = tl.circ ? L : L + 6;
-        tl.P = ADJ_T[var] / tl.T;
-        if (tl.P < 1) return fail(h, PK_E_ARG, "adjoint tile longer than the variant's CTA size");
-        if (tl.P > g.n1) tl.P = g.n1;
-        tl.L = L;
-        tl.halo = 3;
-        tl.xfast = dir == 0;
-        dim3 grid((g.n1 + tl.P - 1) / tl.P, (b.n[dir] + tl.L - 1) / tl.L, g.n2);
-        const size_t smem = 4ull * PH::NV * tl.P * tl.T * sizeof(double);
-        const AdjKernels<PH> k = adj_variant<PH>(var);
-        std::pair<cudaEvent_t, cudaEvent_t> ev;
-        if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
-        k.s2<<<grid, tl.P * tl.T, smem, h->stream>>>(g, tl, ustar, uout, flags, lam_out, lam_in, m1, h->pp, b.dl[dir],
-                                                     h->d_step, apply_fac);
-        PK_CUDA(h, cudaGetLastError());
-        k.s1<<<grid, tl.P * tl.T, smem, h->stream>>>(g, tl, uin, m1, lam_in, h->pp, h->d_step);
-        PK_CUDA(h, cudaGetLastError());
-        if (int rc = ev_end(h, ev)) return fail(h, rc, "cudaEventRecord failed");
-        h->launches += 2;
-        return PK_OK;
+        var = 0;                                  // not stageable here: the tiled default
     }
+    Tile tl;
+    int L = h->adjL[dir] > 0 ? h->adjL[dir] : default_adj_length(dir, b.n[dir], ADJ_T[var]);
+    if (L > b.n[dir]) L = b.n[dir];
+    tl.circ = (L == b.n[dir] && b.n[dir] <= ADJ_T[var]) ? 1 : 0;
+    if (g.seg_len && g.seg_along) {               // stacked instances: one whole segment per tile
+        L = g.seg_len;
+        tl.circ = 1;
+        if (L > ADJ_T[var]) return fail(h, PK_E_ARG, "instance segment longer than the adjoint variant's CTA size");
+    }
+    if (!tl.circ && L > ADJ_T[var] - 6) L = ADJ_T[var] - 6;
+    tl.T = tl.circ ? L : L + 6;
+    tl.P = ADJ_T[var] / tl.T;
+    if (tl.P < 1) return fail(h, PK_E_ARG, "adjoint tile longer than the variant's CTA size");
+    if (tl.P > g.n1) tl.P = g.n1;
+    tl.L = L;
+    tl.halo = 3;
+    tl.xfast = dir == 0;
+    dim3 grid((g.n1 + tl.P - 1) / tl.P, (b.n[dir] + tl.L - 1) / tl.L, g.n2);
+    const size_t smem = 4ull * PH::NV * tl.P * tl.T * sizeof(double);
+    const AdjKernels<PH> k = adj_variant<PH>(var);
+    static bool done[2][NADJ_VARIANT] = {};
+    if (int rc = raise_smem(h, k.s2, &done[0][var])) return rc;
+    if (int rc = raise_smem(h, k.s1, &done[1][var])) return rc;
+    std::pair<cudaEvent_t, cudaEvent_t> ev;
+    if (int rc = ev_begin(h, &ev)) return fail(h, rc, "cudaEventRecord failed");
+    k.s2<<<grid, tl.P * tl.T, smem, h->stream>>>(g, tl, ustar, uout, flags, lam_out, lam_in, m1, h->pp, b.dl[dir],
+                                                 h->d_step, apply_fac);
+    PK_CUDA(h, cudaGetLastError());
+    k.s1<<<grid, tl.P * tl.T, smem, h->stream>>>(g, tl, uin, m1, lam_in, h->pp, h->d_step);
+    PK_CUDA(h, cudaGetLastError());
+    if (int rc = ev_end(h, ev)) return fail(h, rc, "cudaEventRecord failed");
+    h->launches += 2;
+    return PK_OK;
 }
 
 template <class PH, bool FAST = false>
@@ -752,17 +775,26 @@ int launch_unsplit_apply(pk_ctx* h, Block& b, const double* S, double* T, double
 template <class PH>
 const FastOps* make_fast_ops()
 {
-    static FastOps o{set_fused_attr<PH, true>, launch_fused<PH, true>, launch_batched<PH, true>};
+    static FastOps o{set_fused_attr<PH, true>, ready_sweep<PH, true>, launch_fused<PH, true>, launch_batched<PH, true>};
     return &o;
 }
 
 template <class PH>
 const PhysOps* make_ops()
 {
-    static PhysOps o{PH::NV, set_smem_attr<PH>, launch_fused<PH>, launch_open<PH>, launch_stage<PH>,
+    static PhysOps o{PH::NV, set_smem_attr<PH>, ready_sweep<PH>, set_open_attr<PH>, launch_fused<PH>, launch_open<PH>,
+                     launch_stage<PH>,
                      launch_stage_batched<PH>,
-                     launch_stage_refined<PH>, launch_batched<PH>, launch_fused_ptr<PH>, launch_fused_rec<PH>, launch_adj<PH>,
-                     launch_unsplit_flux<PH>, launch_unsplit_apply<PH>};
+                     launch_stage_refined<PH>, launch_batched<PH>, launch_fused_ptr<PH>, launch_unsplit_flux<PH>,
+                     launch_unsplit_apply<PH>};
+    return &o;
+}
+
+// the differentiable path's sweeps of PH (instantiated by the pk_grad_*.cu units only)
+template <class PH>
+const GradOps* make_grad_ops()
+{
+    static GradOps o{launch_fused_rec<PH>, launch_adj<PH>};
     return &o;
 }
 
