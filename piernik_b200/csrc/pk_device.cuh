@@ -180,7 +180,8 @@ PK_PHYS double slope_interior(int lim, double dl, double dr)
 }
 
 // half * f_limiter(q) of an interior cell for a limiter known at compile time
-// (dq_interp = half * f_limiter(q), interpolations.F90:170-204).  Bit for bit
+// (dq_interp = half * f_limiter(q), interpolations.F90:170-204; van Leer's is
+// vanleer_half in pk_quotient.cuh).  Bit for bit
 // 0.5 * slope_interior(LIM, dl, dr): the signs s of minmod, moncen and superbee
 // are -2, 0 or 2, so ((s * m) * 0.5) * 0.5 rounds once, as (s / 4) * m does (for
 // differences below 2^1022 and infinite ones; s = 0 keeps the +0, and the NaN of 0 * inf),
@@ -188,10 +189,7 @@ PK_PHYS double slope_interior(int lim, double dl, double dr)
 template <int LIM>
 PK_PHYS double half_slope(double dl, double dr)
 {
-    if (LIM == L_VANLEER) {
-        const double dcen = dl * dr;
-        return 0.5 * ((dcen > 0.0) ? (2.0 * dcen) / (dl + dr) : 0.0);
-    }
+    static_assert(LIM != L_VANLEER, "van Leer's half slopes are taken in groups");
     const double adl = fabs(dl), adr = fabs(dr);
     double m;
     if (LIM == L_MINMOD) m = f_min(adl, adr);
@@ -233,12 +231,6 @@ PK_PHYS void weno3_faces(A& ar, double qm, double qc, double qp, double weps, do
     f0 = 0.5 * (qc + qm);
     f1 = 0.5 * (-qp + 3.0 * qc);
     qr = w0 * f0 + w1 * f1;
-}
-
-PK_PHYS double slope_end(int lim, double d)
-{
-    if (lim == L_VANLEER) return 0.0;             // "sanitizing endpoints" (:119-120)
-    return slope_interior(lim, d, d);
 }
 
 // -------------------------------------------------------------------------

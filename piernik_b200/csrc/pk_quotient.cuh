@@ -138,6 +138,38 @@ static __device__ __noinline__ void weno3_ieee(double qm, double qc, double qp, 
 
 static __device__ __noinline__ double divide_ieee(double n, double d) { return n / d; }
 
+// Half slopes of van Leer's limiter (0.5 * slope_interior(L_VANLEER, ...): dl dr /
+// (dl + dr) where dl dr > 0, else 0) of a group of G components: their quotients
+// overlap, and a warp in a uniform region skips them together.  Zero at the
+// pencil ends (on: not one).
+// Against an IEEE division per component: unsplit step of a 128^3 MHD block
+// 2.14 -> 2.01 ms, refined blast 23.3 -> 22.8; a 64^3 Sedov blast, at rest
+// almost everywhere, 0.26 either way (without the joint skip 0.28).
+template <int G>
+PK_DEV void vanleer_half(bool on, const double (&dl)[G], const double (&dr)[G], double (&h)[G])
+{
+    double n[G], d[G];
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < G; ++k) {
+        const double dcen = dl[k] * dr[k];
+        const bool up = on && dcen > 0.0;
+        n[k] = up ? 2.0 * dcen : 0.0;
+        d[k] = up ? dl[k] + dr[k] : 1.0;
+        h[k] = 0.0;
+        any = any || up;
+    }
+    if (any) {
+        Exact ar;
+#pragma unroll
+        for (int k = 0; k < G; ++k) h[k] = 0.5 * ar.mean(n[k], d[k]);
+        if (!ar.ok()) {
+#pragma unroll
+            for (int k = 0; k < G; ++k) h[k] = 0.5 * divide_ieee(n[k], d[k]);
+        }
+    }
+}
+
 // n / d, correctly rounded: the floors' quotient
 struct ExactQuotient {
     PK_DEV double operator()(double n, double d) const

@@ -1,6 +1,8 @@
 // Device harness of the branch-free correctly rounded quotients
 // (piernik_b200/csrc/pk_quotient.cuh): quo, quoz, quoc and mean of n operand pairs,
-// whether the operands were in their range, and CUDA's division, for the GPU test.
+// whether the operands were in their range, and CUDA's division; and of van
+// Leer's half slopes of groups of five, next to half of slope_interior, for the
+// GPU test.
 #include <cuda_runtime.h>
 
 #include "../../piernik_b200/csrc/pk_quotient.cuh"
@@ -40,5 +42,42 @@ extern "C" int quotient_eval(const double* n, const double* d, int cnt, double* 
     cudaFree(dn);
     cudaFree(dd);
     cudaFree(dout);
+    return (int)e;
+}
+
+constexpr int G = 5;
+
+__global__ void k_vanleer(int on, const double* dl, const double* dr, int cnt, double* got, double* want)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cnt) return;
+    double a[G], b[G], h[G];
+    for (int k = 0; k < G; ++k) {
+        a[k] = dl[(long long)i * G + k];
+        b[k] = dr[(long long)i * G + k];
+    }
+    pk::vanleer_half(on != 0, a, b, h);
+    for (int k = 0; k < G; ++k) {
+        got[(long long)i * G + k] = h[k];
+        want[(long long)i * G + k] = on ? 0.5 * pk::slope_interior(pk::L_VANLEER, a[k], b[k]) : 0.0;
+    }
+}
+
+// dl, dr, got, want: host arrays of 5 cnt doubles; on = 0: a pencil end; returns a cudaError_t
+extern "C" int vanleer_eval(int on, const double* dl, const double* dr, int cnt, double* got, double* want)
+{
+    const size_t bytes = sizeof(double) * G * (size_t)cnt;
+    double* d[4] = {nullptr, nullptr, nullptr, nullptr};
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < 4 && e == cudaSuccess; ++k) e = cudaMalloc(&d[k], bytes);
+    if (e == cudaSuccess) e = cudaMemcpy(d[0], dl, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d[1], dr, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        k_vanleer<<<(cnt + 255) / 256, 256>>>(on, d[0], d[1], cnt, d[2], d[3]);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(got, d[2], bytes, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(want, d[3], bytes, cudaMemcpyDeviceToHost);
+    for (double* p : d) cudaFree(p);
     return (int)e;
 }

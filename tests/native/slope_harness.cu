@@ -9,8 +9,7 @@ extern "C" void half_slopes(int lim, const double* dl, const double* dr, long lo
 {
     for (long long i = 0; i < n; ++i) {
         want[i] = 0.5 * slope_interior(lim, dl[i], dr[i]);
-        got[i] = lim == L_VANLEER  ? half_slope<L_VANLEER>(dl[i], dr[i])
-                 : lim == L_MINMOD ? half_slope<L_MINMOD>(dl[i], dr[i])
+        got[i] = lim == L_MINMOD   ? half_slope<L_MINMOD>(dl[i], dr[i])
                  : lim == L_MONCEN ? half_slope<L_MONCEN>(dl[i], dr[i])
                                    : half_slope<L_SUPERBEE>(dl[i], dr[i]);
     }

@@ -25,14 +25,18 @@ LIB = os.path.join(HERE, "native", "libquotient_harness.so")
 pytestmark = pytest.mark.gpu
 
 
-def _eval(n, d):
+def _lib():
     if not os.path.exists(LIB) or os.path.getmtime(LIB) < max(os.path.getmtime(p) for p in DEPS):
         subprocess.check_call(["nvcc", "-gencode", "arch=compute_100a,code=sm_100a", "-O3", "--fmad=false",
                                "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-o", LIB, SRC])
+    return C.CDLL(LIB)
+
+
+def _eval(n, d):
     n, d = np.ascontiguousarray(n, float), np.ascontiguousarray(d, float)
     out = np.empty((n.size, 9))
     p = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))  # noqa: E731
-    assert C.CDLL(LIB).quotient_eval(p(n), p(d), n.size, p(out)) == 0
+    assert _lib().quotient_eval(p(n), p(d), n.size, p(out)) == 0
     return out
 
 
@@ -84,6 +88,39 @@ def test_van_leer_mean(gpu_lib):
     assert (zero[:, 8] != 0).all() and (zero[:, 7].copy().view(np.uint64) == 0).all()
     far = _eval([2.0**-950, 2.0**150, np.inf, np.nan, 2.0**100], [2.0**-470, 2.0**100, np.inf, 1.0, np.nan])
     assert (far[:, 8] == 0).all()
+
+
+@pytest.mark.parametrize("on", [1, 0])
+def test_van_leer_half_slopes(gpu_lib, on):
+    """The slopes that the sweeps take (groups of five components, zero at pencil
+    ends) against half of the reference's expression in IEEE operations
+    (fluxlimiters.F90:122-133): random differences, every pair of the edges, and
+    groups of ordinary components with one or two whose operands send the group to
+    its IEEE redo.  The plain slope_interior is the adjoint's and the oracle
+    tests' too."""
+    tiny, sub = np.finfo(float).tiny, np.finfo(float).smallest_subnormal
+    edge = [0.0, sub, 3 * sub, tiny, 1.5 * tiny, 1e-200, 1e-140, 1e-110, 0.75, 1.0, np.nextafter(1.0, 2.0), 3.0, 1e31, 1e120,
+            1e200, 2.0**1022, 2.0**1023, np.inf, np.nan]
+    edge = np.array(edge + [-x for x in edge])
+    rng = np.random.default_rng(10)
+    m = 40000
+    dl = rng.standard_normal((m, 5)) * 10.0 ** rng.integers(-3, 3, (m, 5))
+    dr = np.where(rng.random((m, 5)) < 0.5, dl * (1 + 0.1 * rng.standard_normal((m, 5))), rng.standard_normal((m, 5)))
+    a, b = np.repeat(edge, edge.size), np.tile(edge, edge.size)
+    rows = np.arange(a.size)
+    for k in (0, 3, 4):                    # each pair of edges in a group of ordinary differences
+        dl[k * 8000 + rows, k], dr[k * 8000 + rows, k] = a, b
+    dl[16000 + rows, 1], dr[16000 + rows, 1] = b, b
+    dl[16000 + rows, 2], dr[16000 + rows, 2] = a, b
+    dl[10000:12000], dr[12000:14000] = 0.0, -0.0
+    got, want = np.empty_like(dl), np.empty_like(dl)
+    p = lambda x: x.ctypes.data_as(C.POINTER(C.c_double))  # noqa: E731
+    dl, dr = np.ascontiguousarray(dl), np.ascontiguousarray(dr)
+    assert _lib().vanleer_eval(on, p(dl), p(dr), m, p(got), p(want)) == 0
+    nan = np.isnan(want)
+    assert np.array_equal(nan, np.isnan(got))
+    assert np.array_equal(got[~nan].view(np.uint64), want[~nan].view(np.uint64))
+    assert (want != 0).any() == bool(on)
 
 
 def test_quotients_next_to_a_midpoint(gpu_lib):

@@ -1,4 +1,5 @@
-"""The kernels' limited half slopes against half of the reference's expression
+"""The kernels' limited half slopes (minmod, moncen, superbee; van Leer's is a device
+function, test_gpu_quotient.py) against half of the reference's expression
 (fluxlimiters.F90:109-216), bit for bit, over ordinary differences and the
 edges: signed zeros, subnormals, powers of two and their neighbours,
 infinities and NaN.  The finite values stay below 2^1022: from there on the
@@ -17,7 +18,7 @@ DEP = os.path.join(HERE, "..", "piernik_b200", "csrc", "pk_device.cuh")
 LIB = os.path.join(HERE, "native", "libslope_harness.so")
 
 
-@pytest.mark.parametrize("lim", range(4), ids=["vanleer", "minmod", "moncen", "superbee"])
+@pytest.mark.parametrize("lim", range(1, 4), ids=["minmod", "moncen", "superbee"])
 def test_half_slope_is_half_the_slope(lim):
     if not os.path.exists(LIB) or os.path.getmtime(LIB) < max(os.path.getmtime(SRC), os.path.getmtime(DEP)):
         subprocess.check_call(["nvcc", "-std=c++17", "--fmad=false", "-Xcompiler", "-fPIC,-O2,-ffp-contract=off",
