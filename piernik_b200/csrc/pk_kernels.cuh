@@ -103,20 +103,21 @@ struct Roles {
 // block behind them).  c0: the tile's first owned cell, at position 4.
 PK_PHYS int fused_end(int T, bool wrap, int c0, int n) { return wrap || c0 + T - 4 <= n + 4 ? T : n + 8 - c0; }
 
-// The roles of position t < end in stage 0 or 1 of the fused sweep: each stage
-// uses up two cells at either end, of the cells that are there.  A circular tile
-// (a whole periodic pencil) has no ends.
-PK_PHYS Roles fused_roles(bool active, bool circ, int t, int end, int stage)
+// The roles of position t < end in the fused sweep, four bits a stage (q, slope,
+// flux, upd; one register over the stages): each stage uses up two cells at
+// either end, of the cells that are there.  A circular tile (a whole periodic
+// pencil) has no ends.
+PK_PHYS unsigned fused_roles(bool circ, int t, int end)
 {
-    const int a = 2 * stage;
-    Roles r;
-    r.end = 0;
-    r.keep = false;
-    r.q = active && (circ || (t >= a && t < end - a));
-    r.slope = active && (circ || (t >= a + 1 && t < end - a - 1));
-    r.flux = active && (circ || (t >= a + 1 && t < end - a - 2));
-    r.upd = active && (circ || (t >= a + 2 && t < end - a - 2));
-    return r;
+    if (circ) return 0xffu;
+    unsigned bits = 0;
+    for (int stage = 0; stage < 2; ++stage) {
+        const int a = 2 * stage;
+        const unsigned r = (t >= a && t < end - a ? 1u : 0u) | (t >= a + 1 && t < end - a - 1 ? 2u : 0u) |
+                           (t >= a + 1 && t < end - a - 2 ? 4u : 0u) | (t >= a + 2 && t < end - a - 2 ? 8u : 0u);
+        bits |= r << (4 * stage);
+    }
+    return bits;
 }
 
 // Shared-memory planes of a tile, S doubles per plane (S a compile-time bound
@@ -446,6 +447,7 @@ PK_DEV void fused_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
     const int s = circ ? c0 + t : c0 - 4 + t;                  // position along the pencil (interior coords)
     const int end = fused_end(T, circ || tl.wrap, c0, g.n_d);
     const bool active = (tid < PT) && (i1 < g.n1) && t < end;
+    const unsigned roles = active ? fused_roles(circ, t, end) : 0u;
     const long long off = (long long)(g.g_d + (tl.wrap ? wrap(s, g.n_d) : s)) * g.sd + (long long)(g.g1 + i1) * g.s1 +
                           (long long)(g.g2 + i2) * g.s2;
     const int mp = circ ? p * pstride + (t == 0 ? T - 1 : t - 1) * st : me - st;
@@ -462,7 +464,8 @@ PK_DEV void fused_tile(const Geom& g, const Tile& tl, int i1_0, int c0, int i2, 
     for (int stage = 0; stage < 2; ++stage) {
         // stage 1 (RK2_1) on tile cells [0, end) (circular: every cell); stage 2
         // (RK2_2) on tile cells [2, end-2), u0 again the sweep's input
-        const Roles r = fused_roles(active, circ, t, end, stage);
+        const unsigned bits = roles >> (4 * stage);
+        const Roles r{(bits & 1u) != 0, (bits & 2u) != 0, 0, (bits & 4u) != 0, (bits & 8u) != 0, false};
         FloorRec rec{0, 0};
         rk_stage<PH, S, REC, W3, false, FAST>(smem, me, mp, mn, r, w, uin, uin, off, g, stage == 0 ? dtodx1 : dtodx2, ch,
                                            stp.rch, pp, status, &rec);

@@ -8,11 +8,11 @@ using namespace pk;
 // first owned cell is c0, of a pencil of n cells; returns the tile's end
 extern "C" int fused_tile_roles(int T, int wrap, int circ, int c0, int n, unsigned char* out)
 {
-    const int end = fused_end(T, circ || wrap, c0, n);
+    const int end = fused_end(T, wrap, c0, n);
     for (int stage = 0; stage < 2; ++stage)
         for (int t = 0; t < T; ++t) {
-            const Roles r = fused_roles(t < end, circ, t, end, stage);
-            out[stage * T + t] = (unsigned char)(r.q | r.slope << 1 | r.flux << 2 | r.upd << 3);
+            const unsigned r = t < end ? fused_roles(circ, t, end) : 0u;
+            out[stage * T + t] = (unsigned char)((r >> (4 * stage)) & 15u);
         }
     return end;
 }
