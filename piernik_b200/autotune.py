@@ -84,6 +84,9 @@ def autotune(sim, reps: int = 2, cache: Optional[str] = None, verbose: bool = Fa
         o = [x for x in range(3) if x != d]
         n1 = setup.n[1] if d == 0 else setup.n[0]
         results = []
+        sim.set_tile(d, 0, 0, -1)                # untuned: the tile that the library picks by size
+        sim.sweep(d + 1, dt, ch)                 # its kernel loads at the first launch
+        default_ms = _time_sweep(sim, d, dt, ch, reps)
         for P, Lc, v in candidates(setup.n[d], n1):
             sim.set_tile(d, P, Lc, v)
             ms = _time_sweep(sim, d, dt, ch, reps)
@@ -92,8 +95,7 @@ def autotune(sim, reps: int = 2, cache: Optional[str] = None, verbose: bool = Fa
                 print(f"dir {d} P={P} L={Lc} V={v}: {ms:.3f} ms")
         results.sort()
         ms, P, Lc, v = results[0]
-        best[d] = {"P": P, "L": Lc, "V": v, "ms": ms, "candidates": len(results),
-                   "default_ms": next((r[0] for r in results if (r[1], r[2], r[3]) == (4 if d else 2, min(64, setup.n[d]), 0)), None)}
+        best[d] = {"P": P, "L": Lc, "V": v, "ms": ms, "candidates": len(results), "default_ms": default_ms}
         sim.set_tile(d, P, Lc, v)
     sim.upload(*state, layout=L.PK_LAYOUT_SOA)
     sim.time_state = ts

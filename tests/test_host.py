@@ -151,3 +151,42 @@ def test_missing_library_fails_loudly(tmp_path, monkeypatch):
     monkeypatch.setattr(L, "_lib", None)
     with pytest.raises(L.PkError):
         L.load(str(tmp_path / "absent.so"))
+
+
+def test_autotune_reports_the_untuned_tile():
+    """default_ms is the time of the tile that an untuned run takes (the library's
+    choice by size), and the tuned tile is the fastest candidate's."""
+    from piernik_b200.autotune import autotune, candidates
+
+    class Sim:
+        setup = Setup(n=(128, 128, 128), magnetic=False, fluids=[("neu", 1.4)])
+        time_state = None
+        tile = {}
+
+        def download(self, layout):
+            return ()
+
+        def upload(self, *state, layout):
+            pass
+
+        def timestep_raw(self):
+            return 0.1, 1.0
+
+        def set_tile(self, d, pencils, length, variant=-1):
+            self.tile[d] = (pencils, length, variant)
+
+        def profile(self, on):
+            pass
+
+        def sweep(self, cdim, dt, ch):
+            self.swept = self.tile[cdim - 1]
+
+        def profile_read(self):
+            swept = getattr(self, "swept", None)
+            return 0, 1, {(0, 0, -1): 7.0, fast: 3.0}.get(swept, 5.0)
+
+    fast = list(candidates(128, 128))[11]
+    best = autotune(Sim(), reps=1)
+    for d in range(3):
+        assert best[d]["default_ms"] == 7.0 and best[d]["ms"] == 3.0
+        assert (best[d]["P"], best[d]["L"], best[d]["V"]) == fast == Sim.tile[d]
