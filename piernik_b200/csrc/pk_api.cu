@@ -2040,9 +2040,10 @@ static int unsplit_sweep(pk_ctx* h)
         if (!h->remote.empty()) return fail(h, PK_E_UNSUPPORTED, "the unsplit scheme runs on one rank");
         if (int rc = exchange_prepare(h)) return rc;
     }
+    for (auto& b : h->blocks)
+        if (b.guards_stale)                            // split sweeps before, on the same handle
+            if (int rc = refresh_guards(h, b)) return rc;
     for (auto& b : h->blocks) {
-        if (!h->connected && b.guards_stale)           // split sweeps before, on the same handle
-            if (int rc = fill_guards_block(h, b)) return rc;
         if (!h->connected && !b.uh) PK_CUDA(h, cudaMalloc(&b.uh, sizeof(double) * h->nplanes * b.plane));
         for (int d = 0; d < 3; ++d)
             if (b.n[d] > 1 && !b.flux[d]) PK_CUDA(h, cudaMalloc(&b.flux[d], sizeof(double) * h->nplanes * b.plane));

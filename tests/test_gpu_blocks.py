@@ -144,3 +144,39 @@ def test_overlapping_blocks_are_rejected(gpu_lib):
     with pytest.raises(RuntimeError, match="overlap"):
         sim.update_boundaries()
     sim.close()
+
+
+@pytest.mark.parametrize("phys", ["hd", "mhd"])
+def test_unsplit_step_after_a_split_sweep(gpu_lib, phys):
+    """A fused sweep (pk_sweep) never stores guard cells; the unsplit step that
+    follows on the same handle reads them, so they must be refreshed first: the
+    tiled domain equals the one block."""
+    full = exact_dl(setup_for(phys, n=(24, 20, 16), lim="moncen", solver="unsplit", cfl=0.3, cfl_glm=0.3))
+    u, b, psi = random_state(full, seed=4)
+    one = Simulation(full)
+    one.upload(u, b, psi)
+    sim = None
+    blocks = tiles([8, 16], [20], [16])
+    for n, off in blocks:
+        s = full.replace(n=n, xmin=tuple(full.xmin[d] + off[d] * full.dl[d] for d in range(3)),
+                         xmax=tuple(full.xmin[d] + (off[d] + n[d]) * full.dl[d] for d in range(3)))
+        if sim is None:
+            sim, bid = Simulation(s), 0
+            sim.set_domain(full.n, (True, True, True))
+        else:
+            bid = sim.add_block(s)
+        sim.place_block(bid, off)
+        sim.upload(window(full, u, n, off), window(full, b, n, off), window(full, psi, n, off), block=bid)
+    sim.update_boundaries()
+    for x in (one, sim):
+        x.sweep(2, 1e-3, 1.0)
+        x.run(1)
+        x.sweep(1, 1e-3, 1.0)
+        x.run(1)
+    ref = one.download()
+    for i, (n, off) in enumerate(blocks):
+        for a, r, name in zip(sim.download(block=i), ref, ("u", "b", "psi")):
+            if a is not None:
+                assert_bitexact(interior_of(full.replace(n=n), a, n, (0, 0, 0)), interior_of(full, r, n, off), f"block {i} {name}")
+    one.close()
+    sim.close()
