@@ -1,13 +1,15 @@
 """CPU emulation of the sweep kernels' index arithmetic.
 
 For every launch shape the library can produce for the given block sizes
-(fused tiles of every variant the autotuner tries, the whole-pencil and
-chunked stage tiles), each thread's global offset and every shared-memory
+(fused tiles of every variant the autotuner tries and the ones it picks by size
+for untuned sweeps, the whole-pencil and chunked stage tiles, the tiles with
+boundary rules), each thread's global offset and every shared-memory
 slot it reads are computed exactly as the kernels do and checked to be in
 bounds; owned cells must be updated.  This runs before any GPU sees a new
-tile shape.  Mirrors k_sweep_fused / k_stage / k_stage_batched / k_unsplit_flux in
-piernik_b200/csrc/pk_kernels.cuh and launch_fused / launch_stage /
-launch_unsplit_flux / build_batch in pk_launch.cuh and pk_api.cu.
+tile shape.  Mirrors k_sweep_fused / k_sweep_open / k_stage / k_stage_batched /
+k_unsplit_flux in piernik_b200/csrc/pk_kernels.cuh and default_tile / launch_fused /
+launch_open / launch_stage / launch_unsplit_flux / build_batch in pk_launch.cuh
+and pk_api.cu.
 """
 import pytest
 
@@ -292,9 +294,10 @@ def check_staged(n, nb, d, nv):
     assert (box[0] * 8) % 16 == 0 and all(1 <= b <= 256 for b in box)
     threads = (nd + 31) // 32 * 32
     assert threads <= 256
-    smem_doubles = 5 * nv * nd
-    bar_off = 5 * nv * nd * 8
-    assert bar_off % 8 == 0 and bar_off + 8 <= smem_doubles * 8 + 16
+    stride = 64 if nd <= 64 else 128 if nd <= 128 else 256   # staged_stride: the planes' stride and launch bound
+    assert nd <= stride and threads <= stride
+    bar_off = (2 * nv * nd + 3 * nv * stride) * 8            # staged_smem: the box, the planes, the barrier
+    assert bar_off % 8 == 0 and bar_off + 16 <= 220 * 1024
     st_t, st_p = (1, nd) if d == 0 else (2, 1)
     stored = set()
     nbx = (n1 + 1) // 2
@@ -347,3 +350,92 @@ def test_staged_refused_for_odd_x():
     assert not staged_ok((51, 40, 40), (4, 4, 4), (59, 48, 48), 9, 1)
     assert not staged_ok((50, 40, 40), (3, 3, 3), (56, 46, 46), 9, 2)
     assert not staged_ok((300, 40, 40), (4, 4, 4), (308, 48, 48), 9, 0)
+
+
+# ---------------------------------------------------------------------------
+# the tiles of untuned sweeps (default_tile in pk_launch.cuh)
+# ---------------------------------------------------------------------------
+def default_tiles(n, d):
+    """(P, L, threads) of default_tile where the staged kernel does not run."""
+    G = geom(n, 4, d)
+    if n[0] * n[1] * n[2] < 32768:
+        return (2, 4, 4)[d], 64, 320
+    whole = 256 // n[d]
+    if whole >= 1 if d == 0 else (whole >= 4 or (whole >= 1 and G["n1"] <= whole)):
+        return whole, n[d], 256
+    chunks = -(-n[d] // (88 if d == 0 else 40))
+    return (1 if d == 0 else 4), -(-n[d] // chunks), (128 if d == 0 else 192)
+
+
+@pytest.mark.parametrize("n", CASES + [(33, 33, 33), (63, 64, 65), (258, 16, 12), (12, 16, 258), (89, 41, 25), (300, 130, 1),
+                                       (130, 300, 1), (1, 700, 50), (176, 161, 2)])
+def test_untuned_tiles_indexing(n):
+    for d in range(3):
+        if n[d] > 1:
+            P, L, maxt = default_tiles(n, d)
+            assert (L if L == n[d] else L + 8) <= maxt
+            check_fused(n, d, P, L, maxt)
+
+
+# ---------------------------------------------------------------------------
+# k_sweep_open: whole pencils with their guard cells, whose states are images of
+# interior cells (rules 0 periodic, 1 outflow, 2 reflecting)
+# ---------------------------------------------------------------------------
+OPEN_T = 256
+
+
+def check_open(n, nb, d, lo, hi):
+    G = geom(n, nb, d)
+    nd, g, T = n[d], G["g_d"], G["ext_d"]
+    assert T <= OPEN_T and nd >= g
+    P = min(OPEN_T // T, G["n1"])
+    xfast = d == 0
+
+    def image(x):
+        if 0 <= x < nd:
+            return x, False
+        rule = lo if x < 0 else hi
+        if rule == 0:
+            return (x + nd if x < 0 else x - nd), False
+        if rule == 1:
+            return (0 if x < 0 else nd - 1), False
+        return (-x - 1 if x < 0 else 2 * nd - 1 - x), True
+
+    stored = set()
+    for bx in range((G["n1"] + P - 1) // P):
+        for i2 in range(G["n2"]):
+            for tid in range(P * T):
+                t, p = (tid % T, tid // T) if xfast else (tid // P, tid % P)
+                st = 1 if xfast else P
+                base = tid - t * st
+                i1, s = bx * P + p, t - g
+                if i1 >= G["n1"]:
+                    continue
+                end = -1 if t == 0 else 1 if t == T - 1 else 0
+                cells = [image(x)[0] for x in (s, s + 1 if end < 0 else s - 1, s - 1 if end > 0 else s + 1)]
+                for c in cells:                              # an interior cell's slot, written before it is read
+                    assert 0 <= c < nd and 0 <= base + (c + g) * st < P * T
+                # what the guard refresh would put there (map_guard)
+                if not 0 <= s < nd:
+                    ib = -s if s < 0 else s - nd + 1
+                    want = {0: nd - ib if s < 0 else ib - 1, 1: 0 if s < 0 else nd - 1,
+                            2: ib - 1 if s < 0 else nd - ib}[lo if s < 0 else hi]
+                    assert cells[0] == want and image(s)[1] == ((lo if s < 0 else hi) == 2)
+                off = (g + cells[0]) * G["sd"] + (G["g1"] + i1) * G["s1"] + (G["g2"] + i2) * G["s2"]
+                assert 0 <= off < G["plane"]
+                if end == 0:
+                    assert 0 <= tid - st and tid + st < P * T     # both faces' fluxes
+                if 0 <= s < nd:
+                    assert off not in stored
+                    stored.add(off)
+    assert len(stored) == n[0] * n[1] * n[2]
+
+
+@pytest.mark.parametrize("n,nb", [((12, 10, 8), 4), ((4, 5, 6), 4), ((33, 20, 17), 4), ((248, 5, 4), 4), ((5, 248, 4), 4),
+                                  ((7, 5, 248), 4), ((40, 30, 1), 4), ((250, 6, 6), 3), ((12, 7, 6), 6), ((2, 8, 2), 2)])
+def test_open_kernel_indexing(n, nb):
+    for d in range(3):
+        if n[d] > 1 and nb <= n[d] and n[d] + 2 * nb <= OPEN_T:
+            for lo in range(3):
+                for hi in range(3):
+                    check_open(n, nb, d, lo, hi)
