@@ -218,11 +218,12 @@ int pk_sync(pk_handle h);
 /* Tile shape of the fused sweep for direction d (0..2): P pencils per CTA,
  * L output cells per pencil (the CTA also computes a 4-cell halo each side),
  * and the launch-bound variant (register budget) of the kernel, -1 for the
- * default.  Used by the autotuner; 0 keeps the built-in P / L.  Variant
+ * default.  Used by the autotuner; 0 keeps the built-in P / L, and 0, 0, -1
+ * lets the library pick all three by the block's size (the default).  Variant
  * PK_VARIANT_STAGED sweeps whole pencils (n <= 256) two per CTA, staged in
  * shared memory by TMA bulk-tensor copies (P and L are then ignored); where
- * it cannot run (connected domains, stacked instances, WENO3, odd x extent or
- * guard width) the whole-pencil tile of variant 2 runs instead. */
+ * it cannot run (connected domains, stacked instances along z, WENO3, odd x
+ * extent or guard width) the whole-pencil tile of variant 2 runs instead. */
 #define PK_VARIANT_STAGED 7
 int pk_set_tile(pk_handle h, int32_t dir, int32_t pencils, int32_t length, int32_t variant);
 
@@ -292,9 +293,11 @@ int pk_set_instance_state(pk_handle h, int32_t instance, const pk_time_state* st
  * off on that grid.  From then on every guard refresh (pk_fill_guards, and
  * the one after each RK stage of pk_sweep) copies the neighbours' interior
  * cells into the guard cells that lie over them, after the blocks' own
- * boundary rules (outflow / reflecting) have filled the rest; the sweep runs
- * per RK stage (pk_solve_cg) for such a domain.  Overlapping blocks are
- * rejected at the first refresh. */
+ * boundary rules (outflow / reflecting) have filled the rest (where there is
+ * a rest: not in a domain that the blocks tile and that is periodic in every
+ * direction).  A domain so tiled sweeps with both RK stages in one launch where
+ * it has four guard layers or more, any other per RK stage (pk_solve_cg).
+ * Overlapping blocks are rejected at the first refresh. */
 int pk_set_domain(pk_handle h, const int64_t ncells[3], const int32_t periodic[3]);
 int pk_block_place(pk_handle h, int32_t id, const int64_t off[3]);
 

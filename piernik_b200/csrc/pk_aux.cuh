@@ -321,7 +321,7 @@ __device__ __forceinline__ int map_guard(int i, int n, int g, int side_lo, int s
 
 // Guard cells only, a warp per row along x: of a row that crosses the interior the
 // 2 g_x end cells, 32 / (2 g_x) planes at a time; of any other row every cell,
-// eight planes' loads in flight before their stores (sources are interior cells,
+// nine planes' loads in flight before their stores (sources are interior cells,
 // so nothing written here is read).  Bound by the latency of the scattered 8-byte
 // ends (the bytes are few).  With one thread per cell of the whole block, copying
 // a plane at a time (51 us for a 128^3 MHD block), a step of a 149 x 93 x 70 open

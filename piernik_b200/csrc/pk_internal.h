@@ -18,8 +18,9 @@ namespace pk {
 // the register budget the compiler may use is 65536 / (threads * CTAs);
 // tighter budgets trade spills for resident warps.  The autotuner picks one
 // per direction.
-// Variant VAR_STAGED is the TMA-staged whole-pencil kernel (pk_staged.cuh:
-// two pencils per 256-thread CTA, two CTAs per SM).
+// Variant VAR_STAGED is the TMA-staged whole-pencil kernel (pk_staged.cuh: two
+// pencils per CTA of up to 64, 128 or 256 threads by the pencil's length,
+// 512 threads per SM); its entry in these tables is its largest CTA.
 constexpr int NVARIANT = 8;
 constexpr int VAR_T[NVARIANT] = {320, 256, 256, 128, 128, 192, 512, 256};
 constexpr int VAR_B[NVARIANT] = {1, 1, 2, 3, 4, 2, 1, 2};
@@ -146,7 +147,11 @@ struct pk_ctx {
     long long eglm_plane = 0;
     // launch-bound variant of k_stage_batched (SV_T / SV_B): 384 x 1, twelve warps at 168
     // registers, which hold the solver almost without spills; refined three-fluid
-    // blast per pass 20.6 ms (320 x 1: 22.0, 128 x 3: 24.2, 192 x 2: 21.1)
+    // blast per pass 20.6 ms (320 x 1: 22.0, 128 x 3: 24.2, 192 x 2: 21.1).  Six sweeps
+    // of the same layout with other fluids, 384 x 1 / 320 x 1, ms: MHD 17.1 / 18.6,
+    // MHD + gas 22.8 / 24.5, gas + dust 9.2 / 9.9, gas 7.2 / 7.8 (128 x 3: 6.6); of
+    // connected gas blocks with open walls 8.6 / 9.1 (64 of 32^3), 2.31 / 2.37 (18
+    // uneven ones), 3.85 / 3.83 (64 of 16^3)
     int stage_variant = 3;
     pk::FcArgs* d_fcargs[3] = {nullptr, nullptr, nullptr};   // per block flux couplings (refined domains)
     pk_time_state ts;
