@@ -45,7 +45,7 @@ PK_PHYS void cfl_speeds(A& ar, const CflFluid& fl, double dn, double mx, double 
     }
     cs = 0.0;
     if (fl.kind != K_DST) {
-        const double ek = ar.quoz(0.5 * ((mx * mx + my * my) + mz * mz), dn, r);
+        const double ek = ar.quoa(0.5 * ((mx * mx + my * my) + mz * mz), dn, r, en);
         double c;
         if (fl.kind == K_ION) {
             const double ps = (en - ek) * fl.gam_1 + (2.0 - fl.gam) * pmag;

@@ -110,16 +110,25 @@ enum StatusBits : unsigned {
 // The arithmetic of utoq and of the Riemann solves, passed as a policy (Ieee
 // here; Exact, the kernels', in pk_quotient.cuh; Fast, the tolerance mode's, in
 // pk_fast.cuh).  inv(d) is taken once per denominator and used by every
-// quo(n, d, inv(d)); quoz is quo for numerators that are often exactly zero;
-// quoc divides by a constant d whose correctly rounded reciprocal y is known;
-// root(x, aux) is sqrt(x), and over_root(n, root, aux) is n / that root.  ok()
+// quo(n, d, inv(d)); quoz is quo for numerators that are often exactly zero or
+// fade towards it; quoa is quoz for a quotient that only enters sums with big,
+// quob for one that is only compared with a and b; quoc divides by a constant d
+// whose correctly rounded reciprocal y is known;
+// root(x, aux) is sqrt(x), and over_root(n, root, aux) is n / that root.  settle ends
+// a group of quotients taken with an A of its own.  ok()
 // tells whether all quotients taken so far are the correctly rounded ones.
 struct Ieee {
     static constexpr bool FAST = false;
     PK_PHYS double inv(double) { return 0.0; }
     PK_PHYS double quo(double n, double d, double) { return n / d; }
     PK_PHYS double quoz(double n, double d, double) { return n / d; }
+    PK_PHYS double quoa(double n, double d, double, double) { return n / d; }
+    PK_PHYS double quob(double n, double d, double, double, double) { return n / d; }
     PK_PHYS double quoc(double n, double d, double) { return n / d; }
+    template <int G>
+    PK_PHYS void settle(const double (&)[G], const double (&)[G], double (&)[G])
+    {
+    }
     PK_PHYS double root(double x, double&) { return sqrt(x); }
     PK_PHYS double over_root(double n, double root, double) { return n / root; }
     PK_PHYS bool ok() const { return true; }
@@ -135,12 +144,17 @@ PK_PHYS void utoq(A& ar, const double (&u)[PH::NV], double (&q)[PH::NV], const P
     for (int f = 0; f < PH::NFL; ++f) {
         const int b = PH::beg(f);
         const double dn = u[b], mx = u[b + 1], my = u[b + 2], mz = u[b + 3], r = ar.inv(dn);
+        const double n[4] = {mx, my, mz, PH::has_en(f) ? 0.5 * ((mx * mx + my * my) + mz * mz) : 0.0};
+        const double d[4] = {dn, dn, dn, dn};
+        double x[4] = {ar.quoz(mx, dn, r), ar.quoz(my, dn, r), ar.quoz(mz, dn, r), 0.0};
+        if (PH::has_en(f)) x[3] = ar.quoa(n[3], dn, r, u[b + 4]);
+        ar.settle(n, d, x);
         q[b] = dn;
-        q[b + 1] = ar.quoz(mx, dn, r);
-        q[b + 2] = ar.quoz(my, dn, r);
-        q[b + 3] = ar.quoz(mz, dn, r);
+        q[b + 1] = x[0];
+        q[b + 2] = x[1];
+        q[b + 3] = x[2];
         if (PH::has_en(f)) {
-            const double ek = ar.quoz(0.5 * ((mx * mx + my * my) + mz * mz), dn, r);
+            const double ek = x[3];
             double p = pp.gam_1[f] * (u[b + 4] - ek);
             if (PH::magn(f)) {
                 const double bx = u[PH::IB], by = u[PH::IB + 1], bz = u[PH::IB + 2];
@@ -215,7 +229,7 @@ PK_PHYS void weno3_faces(A& ar, double qm, double qc, double qp, double weps, do
     const double tt = ((qp - 2.0 * qc) + qm);                                   // Eq. 22
     const double tau = tt * tt;
     const double e0 = weps + b0, e1 = weps + b1;
-    const double t0 = ar.quoz(tau, e0, ar.inv(e0)), t1 = ar.quoz(tau, e1, ar.inv(e1));
+    const double t0 = ar.quoa(tau, e0, ar.inv(e0), 1.0), t1 = ar.quoa(tau, e1, ar.inv(e1), 1.0);
     double a0 = d0 * (1.0 + t0);                                                // Eq. 21
     double a1 = d1 * (1.0 + t1);
     double s = a0 + a1, r = ar.inv(s);
@@ -345,14 +359,20 @@ PK_PHYS void hlld_face(A& ar, bool has_energy, double gamma, double rgam_1, doub
             sm = (sl + sr) * 0.5;
         } else {
             if constexpr (A::FAST) sm = ar.div(n, d);
-            else sm = ar.quoz(n, d, ar.inv(d));
+            else {
+                A g;
+                const double gn[1] = {n}, gd[1] = {d};
+                double x[1] = {g.quoz(n, d, g.inv(d))};
+                g.settle(gn, gd, x);
+                sm = x[0];
+            }
         }
     }
     const double slsm = sl - sm, srsm = sr - sm;                                    // :334-340
     const double b_lr = bl[0] * br[0];
     double b_lrgam;
     if constexpr (A::FAST) b_lrgam = b_lr * rgam;
-    else b_lrgam = ar.quoc(b_lr, gamma, rgam);
+    else b_lrgam = ar.quob(b_lr, gamma, rgam, ul[4], ur[4]);
     prt_star = 0.5 * ((prl + dn_l * (sm - ul[1])) + (prr + dn_r * (sm - ur[1])));
     // rho*, transverse B* (HLL fallback) and v* of both sides (:354-355, :362-382)
     const double rslsm = ar.inv(slsm), rsrsm = ar.inv(srsm);
@@ -363,6 +383,7 @@ PK_PHYS void hlld_face(A& ar, bool has_energy, double gamma, double rgam_1, doub
         const bool star_l = (fabs(cl) > f_spacing(b_lr)) && b_lrgam <= (has_energy ? ul[4] : 0.0);
         const bool star_r = (fabs(cr) > f_spacing(b_lr)) && b_lrgam <= (has_energy ? ur[4] : 0.0);
         const double tl = dn_l * slvxl - b_lr, tr = dn_r * srvxr - b_lr;
+        double kl = 0.0, kr = 0.0;
         if constexpr (A::FAST) {
             const double ql = ar.div(tl, cl), qr = ar.div(tr, cr);
 #pragma unroll
@@ -371,13 +392,21 @@ PK_PHYS void hlld_face(A& ar, bool has_energy, double gamma, double rgam_1, doub
                 bsr[c] = br[1 + c] * qr;
             }
         } else {
+            A g;
             const double dl = star_l ? cl : 1.0, dr = star_r ? cr : 1.0;
-            const double rl = ar.inv(dl), rr = ar.inv(dr);
+            const double rl = g.inv(dl), rr = g.inv(dr);
+            const double n[6] = {bl[1] * tl, bl[2] * tl, br[1] * tr, br[2] * tr, bl[0], br[0]};
+            const double d[6] = {dl, dl, dr, dr, dn_l, dn_r};
+            double x[6] = {g.quoz(n[0], dl, rl), g.quoz(n[1], dl, rl), g.quoz(n[2], dr, rr), g.quoz(n[3], dr, rr),
+                           g.quoz(n[4], dn_l, g.inv(dn_l)), g.quoz(n[5], dn_r, g.inv(dn_r))};
+            g.settle(n, d, x);
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                bsl[c] = ar.quoz(bl[1 + c] * tl, dl, rl);
-                bsr[c] = ar.quoz(br[1 + c] * tr, dr, rr);
+                bsl[c] = x[c];
+                bsr[c] = x[2 + c];
             }
+            kl = x[4];
+            kr = x[5];
         }
         if (!(star_l && star_r)) {
             const double d = sr - sl, r = ar.inv(d);
@@ -388,13 +417,9 @@ PK_PHYS void hlld_face(A& ar, bool has_energy, double gamma, double rgam_1, doub
                 if (!star_r) bsr[c] = h;
             }
         }
-        double kl, kr;
         if constexpr (A::FAST) {
             kl = ar.div(bl[0], dn_l);
             kr = ar.div(br[0], dn_r);
-        } else {
-            kl = ar.quoz(bl[0], dn_l, ar.inv(dn_l));
-            kr = ar.quoz(br[0], dn_r, ar.inv(dn_r));
         }
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -408,20 +433,37 @@ PK_PHYS void hlld_face(A& ar, bool has_energy, double gamma, double rgam_1, doub
         double xl = 0.0, xr = 0.0;
         rtl = ar.root(usl0, xl);
         rtr = ar.root(usr0, xr);
-        alfven_l = sm - ar.over_root(fabs(bl[0]), rtl, xl);
-        alfven_r = sm + ar.over_root(fabs(br[0]), rtr, xr);
+        {
+            A g;
+            const double n[2] = {fabs(bl[0]), fabs(br[0])}, d[2] = {rtl, rtr};
+            double x[2] = {g.over_root(n[0], rtl, xl), g.over_root(n[1], rtr, xr)};
+            g.settle(n, d, x);
+            alfven_l = sm - x[0];
+            alfven_r = sm + x[1];
+        }
         alfven = !(alfven_l > 0.0 || alfven_r < 0.0);
         if (!alfven) {
             left = alfven_l > 0.0;
             both = false;
         } else {                                                                     // :452-470
             const double b_sig = (bl[0] >= 0.0) ? 1.0 : -1.0;
-            const double d = rtl + rtr, r = ar.inv(d), bsm = b_sig * (rtl * rtr);
+            A g;
+            const double d = rtl + rtr, r = g.inv(d), bsm = b_sig * (rtl * rtr);
             b2n = 0.5 * (bl[0] + br[0]);
+            double n[4], x[4];
+            const double ds[4] = {d, d, d, d};
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                v2[c] = ar.quoz((rtl * vsl[c] + rtr * vsr[c]) + b_sig * (bsr[c] - bsl[c]), d, r);
-                b2[c] = ar.quoz((rtl * bsr[c] + rtr * bsl[c]) + bsm * (vsr[c] - vsl[c]), d, r);
+                n[c] = (rtl * vsl[c] + rtr * vsr[c]) + b_sig * (bsr[c] - bsl[c]);
+                n[2 + c] = (rtl * bsr[c] + rtr * bsl[c]) + bsm * (vsr[c] - vsl[c]);
+                x[c] = g.quoz(n[c], d, r);
+                x[2 + c] = g.quoz(n[2 + c], d, r);
+            }
+            g.settle(n, ds, x);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                v2[c] = x[c];
+                b2[c] = x[2 + c];
             }
         }
     }
@@ -479,7 +521,13 @@ PK_PHYS void hllc_face(A& ar, bool has_energy, double gamma, double rgam_1, cons
             sm = (sl + sr) * 0.5;
         } else {
             if constexpr (A::FAST) sm = ar.div(n, d);
-            else sm = ar.quoz(n, d, ar.inv(d));
+            else {
+                A g;
+                const double gn[1] = {n}, gd[1] = {d};
+                double x[1] = {g.quoz(n, d, g.inv(d))};
+                g.settle(gn, gd, x);
+                sm = x[0];
+            }
         }
         prt_star = 0.5 * ((prl + dn_l * (sm - ul[1])) + (prr + dn_r * (sm - ur[1])));
         left = !(sm < 0.0);
@@ -581,10 +629,13 @@ PK_PHYS void riemann(const double (&ql)[PH::NV], const double (&qr)[PH::NV], dou
 }
 
 // internal_sources (+0 added to every fluid component) and care_for_positives
-// on one updated cell; B used for emag is the updated one (b1).  quotient(n, d):
-// n / d, correctly rounded.
+// on one updated cell; B used for emag is the updated one (b1).  quotient(n, d, big):
+// n / d, correctly rounded unless a positive energy big absorbs it.  (It does: the
+// kinetic energy enters u - kin and, with the floored internal energy, e + kin.
+// Where u > 0 and 2^62 kin < u, u - kin = u; for a magnetised fluid whose field
+// energy cancels u the sum with that energy follows and absorbs it.)
 struct IeeeQuotient {
-    PK_PHYS double operator()(double n, double d) const { return n / d; }
+    PK_PHYS double operator()(double n, double d, double) const { return n / d; }
 };
 
 template <class PH, class Quotient = IeeeQuotient>
@@ -603,7 +654,8 @@ PK_PHYS void sources_and_floors(double (&u)[PH::NV], const PhysParams& pp, unsig
     for (int f = 0; f < PH::NFL; ++f) {                                   // limit_minimal_intener
         if (!PH::has_en(f)) continue;
         const int b = PH::beg(f);
-        const double kin = quotient(0.5 * ((u[b + 1] * u[b + 1] + u[b + 2] * u[b + 2]) + u[b + 3] * u[b + 3]), u[b]);
+        const double kin = quotient(0.5 * ((u[b + 1] * u[b + 1] + u[b + 2] * u[b + 2]) + u[b + 3] * u[b + 3]), u[b],
+                                    u[b + 4] > 0.0 ? u[b + 4] : 0.0);
         double mag = 0.0, eint;
         if (PH::magn(f)) {
             const double bx = u[PH::IB], by = u[PH::IB + 1], bz = u[PH::IB + 2];
@@ -649,7 +701,8 @@ PK_PHYS void floors_rec(double (&u)[PH::NV], const PhysParams& pp, unsigned& sta
     for (int f = 0; f < PH::NFL; ++f) {
         if (!PH::has_en(f)) continue;
         const int b = PH::beg(f);
-        const double kin = quotient(0.5 * ((u[b + 1] * u[b + 1] + u[b + 2] * u[b + 2]) + u[b + 3] * u[b + 3]), u[b]);
+        const double kin = quotient(0.5 * ((u[b + 1] * u[b + 1] + u[b + 2] * u[b + 2]) + u[b + 3] * u[b + 3]), u[b],
+                                    u[b + 4] > 0.0 ? u[b + 4] : 0.0);
         double mag = 0.0, eint;
         if (PH::magn(f)) {
             const double bx = u[PH::IB], by = u[PH::IB + 1], bz = u[PH::IB + 2];

@@ -102,6 +102,10 @@ struct Fast {
         return x * y;
     }
     PK_DEV double over_root(double n, double, double y) { return n * y; }
+    template <int G>
+    PK_DEV void settle(const double (&)[G], const double (&)[G], double (&)[G]) const
+    {
+    }
     PK_DEV bool ok() const { return true; }
 };
 
@@ -135,7 +139,8 @@ PK_DEV void riemann_cell(double (&q)[PH::NV], const double* R, double* F, double
             dps = (psr - psl) * rch;
         } else {
             Exact ar;
-            dps = ar.quoc(psr - psl, ch, rch);
+            ar.needd(ch);
+            dps = ar.quoa(psr - psl, ch, rch, bxr + bxl);
             if (!ar.ok()) dps = divide_ieee(psr - psl, ch);
         }
         put(PH::IB + 3, ((ch * ch) * 0.5) * ((bxr + bxl) - dps));                // hlld.F90:229 (Dedner eq. 42)

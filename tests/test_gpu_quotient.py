@@ -1,9 +1,9 @@
 """The bit-exact kernels' branch-free quotients (pk_quotient.cuh) against
 CUDA's correctly rounded division, bit for bit, wherever they say that the
 operands are in their range, and that they say so for numerators in
-[2^-768, 2^256), denominators in [2^-260, 2^252) and zero numerators of quoz
-and quoc.  Van Leer's mean 2 a b / (a + b) (mean) alike, for 2 a b in [2^-900, 2^124)
-and a + b < 2^100.
+[2^-768, 2^256), denominators in [2^-260, 2^252) and zero numerators of quoz and quoc.  Van Leer's
+mean 2 a b / (a + b) (mean) alike, for a + b < 2^100 and a normal result.  Below these
+ranges the sums that quoa and the comparisons that quob are for.
 
 Operands: random ones; divisors with significands at either end; quotients
 as close to the midpoint of two doubles as they get (n 2^54 - d m = +-1 for an
@@ -74,6 +74,32 @@ def test_far_ends_of_the_range(gpu_lib):
     _check(n, d, True)
 
 
+def test_absorbed_quotients(gpu_lib):
+    """big - x, big + x and x <= big with x of quoa and quob are those with n / d,
+    wherever they say so; and they say so for every small numerator next to an
+    ordinary big, zeros among them."""
+    rng = np.random.default_rng(12)
+    m = 1 << 19
+    n = np.ldexp(1 + rng.random(m), rng.integers(-1080, 20, m)) * rng.choice([-1.0, 0.0, 1.0, 1.0], m)
+    d = np.ldexp(1 + rng.random(m), rng.integers(0, 40, m))
+    big = np.ldexp(1 + rng.random(m), rng.integers(-800, 200, m)) * rng.choice([-1.0, 1.0], m)
+    near = rng.random(m) < 0.3              # quotients about as large as big
+    big = np.where(near, n / d * (1 + rng.integers(-3, 4, m) * 2.0**-52), big)
+    ends = rng.random(m) < 0.2              # powers of two: half the spacing below them
+    big = np.where(ends & ~near, np.ldexp(1.0, rng.integers(-500, 200, m)), big)
+    out = np.empty((m, 8))
+    p = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))  # noqa: E731
+    n, d, big = (np.ascontiguousarray(x) for x in (n, d, big))
+    assert _lib().absorbed_eval(p(n), p(d), p(big), m, p(out)) == 0
+    ok = out[:, 2] != 0
+    for k in (0, 1):
+        assert np.array_equal(out[ok, k].copy().view(np.uint64), out[ok, 3 + k].copy().view(np.uint64)), k
+    okb = out[:, 6] != 0
+    assert np.array_equal(out[okb, 5], out[okb, 7])
+    plain = (np.abs(big) > 2.0**-430) & (np.abs(big) < 2.0**200)
+    assert ok[plain].all() and okb[plain].all() and ok.mean() > 0.5
+
+
 def test_van_leer_mean(gpu_lib):
     rng = np.random.default_rng(9)
     m = 1 << 18
@@ -86,8 +112,17 @@ def test_van_leer_mean(gpu_lib):
     assert np.array_equal(o[:, 7].copy().view(np.uint64), o[:, 6].copy().view(np.uint64))
     zero = _eval(np.zeros(4), np.ones(4))
     assert (zero[:, 8] != 0).all() and (zero[:, 7].copy().view(np.uint64) == 0).all()
-    far = _eval([2.0**-950, 2.0**150, np.inf, np.nan, 2.0**100], [2.0**-470, 2.0**100, np.inf, 1.0, np.nan])
+    # (2^-950 over 2^-470 was refused while products went down to 2^-900 only)
+    far = _eval([2.0**-1060, 2.0**150, np.inf, np.inf, 2.0**100], [2.0**-30, 2.0**100, np.inf, np.nan, np.nan])
     assert (far[:, 8] == 0).all()
+    # products down to the smallest subnormal ones, results down to the smallest normal ones
+    a = np.ldexp(1 + rng.random(m), rng.integers(-537, -400, m))
+    b = np.where(rng.random(m) < 0.5, a * (1 + rng.random(m)), np.ldexp(1 + rng.random(m), rng.integers(-537, -500, m)))
+    n, d = 2.0 * (a * b), a + b
+    o = _eval(n, d)
+    some = n != 0
+    assert (o[some, 8] != 0).all() and some.sum() > m // 2
+    assert np.array_equal(o[some, 7].copy().view(np.uint64), o[some, 6].copy().view(np.uint64))
 
 
 @pytest.mark.parametrize("on", [1, 0])
@@ -95,8 +130,8 @@ def test_van_leer_half_slopes(gpu_lib, on):
     """The slopes that the sweeps take (groups of five components, zero at pencil
     ends) against half of the reference's expression in IEEE operations
     (fluxlimiters.F90:122-133): random differences, every pair of the edges, and
-    groups of ordinary components with one or two whose operands send the group to
-    its IEEE redo.  The plain slope_interior is the adjoint's and the oracle
+    groups of ordinary components with one or two whose operands (beyond 2^100, or
+    with a subnormal result) send the group to its IEEE redo.  The plain slope_interior is the adjoint's and the oracle
     tests' too."""
     tiny, sub = np.finfo(float).tiny, np.finfo(float).smallest_subnormal
     edge = [0.0, sub, 3 * sub, tiny, 1.5 * tiny, 1e-200, 1e-140, 1e-110, 0.75, 1.0, np.nextafter(1.0, 2.0), 3.0, 1e31, 1e120,

@@ -3,7 +3,7 @@ quotients (pk_quotient.cuh) are proven: the threads that hold them redo their
 cells in IEEE operations, and the result must be the oracle's, bit for bit.
 
 Units scaled far down and far up, and fields that fade through the whole
-exponent range (values from 1e-100 to 1e-300 between ordinary ones, so that
+exponent range (values from 1e-100 to 1e-322 between ordinary ones, so that
 some threads of a warp redo their cells and others do not)."""
 import numpy as np
 import pytest
@@ -25,10 +25,10 @@ def scaled(setup, how, seed=3):
             if kind == "dst":
                 continue
             o = sum(4 if k == "dst" else 5 for k, _ in setup.fluids[:f])
-            tiny = 10.0 ** rng.uniform(-300, -100, u.shape[:3] + (3,)) * rng.choice([-1.0, 0.0, 1.0], u.shape[:3] + (3,))
+            tiny = 10.0 ** rng.uniform(-322, -100, u.shape[:3] + (3,)) * rng.choice([-1.0, 0.0, 1.0], u.shape[:3] + (3,))
             u[..., o + 1:o + 4] = np.where(rng.random(u.shape[:3] + (1,)) < 0.7, tiny, u[..., o + 1:o + 4])
         if setup.magnetic:
-            small = 10.0 ** rng.uniform(-300, -100, b.shape) * rng.choice([-1.0, 0.0, 1.0], b.shape)
+            small = 10.0 ** rng.uniform(-322, -100, b.shape) * rng.choice([-1.0, 0.0, 1.0], b.shape)
             b[...] = np.where(rng.random(b.shape) < 0.6, small, b)
         return u, b, psi
     r = {"down": 2.0**-460, "up": 2.0**460}[how]      # densities, momenta, energies; fields by the root
