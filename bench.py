@@ -43,16 +43,16 @@ NVAR = 9                         # dn, mx, my, mz, en, Bx, By, Bz, psi
 # DRAM bytes per cell of one sweep launch, from one ncu capture
 # (dram__bytes_read.sum + dram__bytes_write.sum) of the TMA-staged y sweep of a
 # 128^3 block (181 MB with guards, above the 126 MB L2) in the tolerance
-# arithmetic: 161.17 MB read + 114.47 MB written over 128^3 cells.  Traffic
+# arithmetic: 160.95 MB read + 111.76 MB written over 128^3 cells.  Traffic
 # grows with the cell count, so the full-size figure is this times n^3.
-TRAFFIC_BYTES_PER_CELL = (161.174272e6 + 114.471424e6) / 128 ** 3
+TRAFFIC_BYTES_PER_CELL = (160.951296e6 + 111.762432e6) / 128 ** 3
 # FP64 flops per cell of one sweep (both RK2 stages) without halo
 # recomputation: 2 x DFMA + DMUL + DADD thread instructions (ncu
 # sm__sass_thread_inst_executed_op_{dfma,dmul,dadd}_pred_on.sum) of the
 # TMA-staged whole-pencil x sweep of a 128^3 block over its 128^3 cells, in
-# the bit-exact arithmetic (0.6356 G DFMA, 0.7657 G DMUL, 0.9212 G DADD) and in
+# the bit-exact arithmetic (0.6356 G DFMA, 0.7735 G DMUL, 0.9269 G DADD) and in
 # the tolerance arithmetic (0.6582 G DFMA, 0.4596 G DMUL, 0.5226 G DADD)
-FP64_FLOP_PER_CELL_SWEEP = (2 * 635607066 + 765703155 + 921207132) / 128 ** 3
+FP64_FLOP_PER_CELL_SWEEP = (2 * 635607066 + 773470185 + 926877010) / 128 ** 3
 FP64_FLOP_PER_CELL_SWEEP_FMA = (2 * 658212674 + 459563829 + 522622051) / 128 ** 3
 ARITH_NOTE = {
     "fma": "fma: multiply-add contraction and hoisted reciprocals in the fused sweep; agrees with the "
