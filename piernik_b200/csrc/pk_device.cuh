@@ -113,10 +113,10 @@ enum StatusBits : unsigned {
 // quo(n, d, inv(d)); quoz is quo for numerators that are often exactly zero or
 // fade towards it; quoa is quoz for a quotient that only enters sums with big,
 // quob for one that is only compared with a and b; quoc divides by a constant d
-// whose correctly rounded reciprocal y is known;
-// root(x, aux) is sqrt(x), and over_root(n, root, aux) is n / that root.  settle ends
-// a group of quotients taken with an A of its own.  ok()
-// tells whether all quotients taken so far are the correctly rounded ones.
+// whose correctly rounded reciprocal y is known; root(x, aux) is sqrt(x), and
+// over_root(n, root, aux) is n / that root.  settle ends a group of quotients taken
+// with an A of its own.  ok() tells whether all quotients taken so far are the
+// correctly rounded ones.
 struct Ieee {
     static constexpr bool FAST = false;
     PK_PHYS double inv(double) { return 0.0; }
